@@ -338,7 +338,7 @@ def run_ours(a):
         if group is not None:
             return parallel.nsa_forward_head_parallel(Q, K, V, cfg, gate_logits=G, group=group)
         return nsa.nsa_forward(Q, K, V, cfg, gate_logits=G)
-    LAUNCHES_PER_STEP = 6   # pool Q means, pool K means, select, pool K, pool V, fused attention
+    LAUNCHES_PER_STEP = 3   # window means of Q, K and V; select; fused attention
 
     for _ in range(a.warmup):
         out = step()
@@ -558,7 +558,7 @@ def run_cp(a, T, nsa, cfg, rank, world, dist, barrier, max_over_ranks, steps, wa
                    "global_batch": 1, "seq_len": T, "parallelism": f"cp{world}: all-gather of K/V ({kv_bytes} B received per rank per step) + local forward",
                    "l2": "inputs exceed the 126 MB L2"},
         "roofline": None, "cpu_baseline": None, "e2e": None, "clocks": clocks,
-        "gpu_launches": 6 * steps,
+        "gpu_launches": 5 * steps,
     }
     del Q, K, V, G, out
     torch.cuda.empty_cache()

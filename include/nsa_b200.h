@@ -200,6 +200,28 @@ typedef struct nsa_fwd_args {
  * nsa_forward (nsa/triton/forward.py:362-406). */
 int nsa_attention_fwd(const nsa_fwd_args* args, nsa_stream_t stream);
 
+/* The whole forward in one call: window means, block selection (unless idx is given), and the fused launch of the
+ * three branches.  Tensors as for nsa_attention_fwd with branches = 7, fused = 1; K/V have Q's type (fp8 included).
+ * has_idx != 0: block lists idx [B,Hi,nq,top_k], Hi = H or Hkv; otherwise they are chosen as nsa_select_blocks does
+ * (top_k, force_first, force_local, per_group).  ws: nsa_forward_ws_bytes(&args) bytes of device memory, 256-byte
+ * aligned, contents free; the sizes alone decide the amount, the pointers may still be NULL when it is asked for
+ * (a negative status instead of a size: bad arguments).
+ * Replaces: nsa_forward, nsa/triton/forward.py:362-406, together with _resolve_block_indices (:321-359). */
+typedef struct nsa_forward_args {
+  const void *Q, *K, *V, *gates;
+  const int32_t* idx;
+  void *out, *ws;
+  int64_t ws_bytes;
+  int32_t B, H, Hkv, Hi, Tq, Tk, D;
+  int32_t has_idx, top_k, force_first, force_local, per_group;
+  int32_t cmp_block, cmp_stride, bm, bn, window, causal;
+  int32_t gate_act, q_dtype, gate_dtype, engine, io_layout;
+  float scale, q_scale, k_scale, v_scale;
+} nsa_forward_args;
+
+int64_t nsa_forward_ws_bytes(const nsa_forward_args* args);
+int nsa_forward(const nsa_forward_args* args, nsa_stream_t stream);
+
 /* Synchronises `stream`, then reports whether any kernel launched so far gave up on one of
  * its bounded device-side waits: NSA_OK, or NSA_ERR_DEVICE (and the condition is cleared).
  * No counterpart in the reference (its kernels have no device-side waits). */

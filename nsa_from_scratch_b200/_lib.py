@@ -72,6 +72,21 @@ class BwdArgs(C.Structure):
     ]
 
 
+class ForwardArgs(C.Structure):
+    """Mirror of `struct nsa_forward_args`."""
+    _fields_ = [
+        ("Q", C.c_void_p), ("K", C.c_void_p), ("V", C.c_void_p), ("gates", C.c_void_p), ("idx", C.c_void_p),
+        ("out", C.c_void_p), ("ws", C.c_void_p), ("ws_bytes", C.c_int64),
+        ("B", C.c_int32), ("H", C.c_int32), ("Hkv", C.c_int32), ("Hi", C.c_int32),
+        ("Tq", C.c_int32), ("Tk", C.c_int32), ("D", C.c_int32),
+        ("has_idx", C.c_int32), ("top_k", C.c_int32), ("force_first", C.c_int32), ("force_local", C.c_int32), ("per_group", C.c_int32),
+        ("cmp_block", C.c_int32), ("cmp_stride", C.c_int32), ("bm", C.c_int32), ("bn", C.c_int32),
+        ("window", C.c_int32), ("causal", C.c_int32),
+        ("gate_act", C.c_int32), ("q_dtype", C.c_int32), ("gate_dtype", C.c_int32), ("engine", C.c_int32), ("io_layout", C.c_int32),
+        ("scale", C.c_float), ("q_scale", C.c_float), ("k_scale", C.c_float), ("v_scale", C.c_float),
+    ]
+
+
 _vp, _i, _f, _i64 = C.c_void_p, C.c_int, C.c_float, C.c_int64
 
 PROTOTYPES = {
@@ -85,6 +100,8 @@ PROTOTYPES = {
     "nsa_cmp_block_scores_tc": (_i, [_vp, _vp, _vp, _vp, _vp] + [_i] * 13 + [_f, _i, _i, _i, _i, _vp]),
     "nsa_topk_from_scores": (_i, [_vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp]),
     "nsa_attention_fwd": (_i, [C.POINTER(FwdArgs), _vp]),
+    "nsa_forward_ws_bytes": (_i64, [C.POINTER(ForwardArgs)]),
+    "nsa_forward": (_i, [C.POINTER(ForwardArgs), _vp]),
     "nsa_device_status": (_i, [_vp]),
     "nsa_debug_set_device_status": (_i, [_i, _i]),
     "nsa_compressed_attention_static": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp]),
@@ -139,7 +156,26 @@ def check(rc: int, what: str) -> None:
 
 
 def stream_ptr(device=None) -> int:
+    if device is None:
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())   # no Stream object on the way
     return torch.cuda.current_stream(device).cuda_stream
+
+
+class _NoGuard:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NO_GUARD = _NoGuard()
+
+
+def on_device(t):
+    """Context in which `t`'s device is current.  Almost every call finds it current already, and entering
+    torch.cuda.device costs several microseconds of a short launch."""
+    return _NO_GUARD if t.device.index == torch.cuda.current_device() else torch.cuda.device(t.device)
 
 
 def ptr(t) -> int:

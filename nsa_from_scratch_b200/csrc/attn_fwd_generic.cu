@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(NW * 32, D <= 64 ? 4 : 2) attn_fwd_generic_ker
   const size_t kc_slab = ((size_t)(b * a.Hkv + hk) * a.Nc) * D;
 
   // ---- stage Q, build the list of selected blocks -------------------------------
+  grid_dep_wait();
   if constexpr (IN8) {
     stage_tile8<D, NT>(Qs, reinterpret_cast<const uint8_t*>(a.Q) + q_slab, q0, TM, a.Tq, a.q_scale, a.q_dtype);
   } else {
@@ -391,8 +392,7 @@ static int launch_generic(const FwdK& k, cudaStream_t st) {
   NSA_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   long long blocks = (long long)k.a.B * k.a.H * k.n_qtiles;
   NSA_REQUIRE(blocks > 0 && blocks < 2147483647LL, NSA_ERR_ARG, "attention forward: %lld tiles do not fit a grid", blocks);
-  fn<<<(unsigned)blocks, NW * 32, smem, st>>>(k);
-  return launch_status("attn_fwd_generic");
+  return launch_pdl("attn_fwd_generic", fn, dim3((unsigned)blocks), NW * 32, smem, st, k);
 }
 
 template <typename T, bool IN8>

@@ -1567,6 +1567,7 @@ __global__ void __launch_bounds__(256) nsa_split_combine_kernel(const float* __r
                                                                 int io_layout, int H, int Tq, long long rows, int nsplit,
                                                                 float os0, float os1, float os2) {
   constexpr int CPT = D / 32;
+  grid_dep_wait();
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);     // (b, h, t) order
   if (row >= rows) return;
@@ -1816,19 +1817,16 @@ int attention_fwd_tc5(const nsa_fwd_args& a, cudaStream_t st) {
     else if (a.D == 128) NSA_TC5_LAUNCH(128, 0, false, true)
     else if (fmt == 1) NSA_TC5_LAUNCH(64, 1, false, true)
     else NSA_TC5_LAUNCH(64, 0, false, true)
-    int rc2 = launch_status("attn_fwd_tc5 (split)");
-    if (rc2 != NSA_OK) return rc2;
+    if ((rc = launch_status("attn_fwd_tc5 (split)")) != NSA_OK) return rc;
     const unsigned cgrid = (unsigned)((rows + 7) / 8);
 #define NSA_TC5_COMBINE(TT, DD)                                                                                        \
-    nsa_split_combine_kernel<TT, DD><<<cgrid, 256, 0, st>>>(p.part, reinterpret_cast<TT*>(a.out), a.gates, a.gate_dtype, \
-                                                            a.gate_act, a.io_layout, a.H, a.Tq, rows, p.nsplit,       \
-                                                            p.out_scale[0], p.out_scale[1], p.out_scale[2])
+    return launch_pdl("split_combine", nsa_split_combine_kernel<TT, DD>, dim3(cgrid), 256, 0, st, p.part, reinterpret_cast<TT*>(a.out), \
+                      a.gates, a.gate_dtype, a.gate_act, a.io_layout, a.H, a.Tq, rows, p.nsplit, p.out_scale[0], p.out_scale[1], p.out_scale[2])
     if (a.D == 128 && fmt == 1) NSA_TC5_COMBINE(__nv_bfloat16, 128);
     else if (a.D == 128) NSA_TC5_COMBINE(__half, 128);
     else if (fmt == 1) NSA_TC5_COMBINE(__nv_bfloat16, 64);
     else NSA_TC5_COMBINE(__half, 64);
 #undef NSA_TC5_COMBINE
-    return launch_status("split_combine");
   }
   const int n_br = ((a.branches >> 0) & 1) + ((a.branches >> 1) & 1) + ((a.branches >> 2) & 1);
   if (!in8 && (tc5_persistent_mode() == 1 || (tc5_persistent_mode() == -1 && n_br == 1))) {

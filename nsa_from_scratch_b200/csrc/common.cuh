@@ -32,6 +32,41 @@ static inline int launch_status(const char* what) {
   return NSA_OK;
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// A kernel launched through launch_pdl may become resident while the kernel before it in the stream is still running,
+// which takes the launch latency and its own set-up off the path between the two.  It must execute grid_dep_wait()
+// before its first access to global memory (reads, and writes to memory an earlier kernel may still read): that waits
+// for the whole kernel before it, and -- because every kernel of the chain waits the same way -- for all before that.
+// grid_dep_launch() lets the next kernel of the stream become resident early; what it waits for does not change.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+static inline int launch_pdl(const char* what, void (*kernel)(KArgs...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  if (e != cudaSuccess) return fail(NSA_ERR_CUDA, "%s launch failed: %s", what, cudaGetErrorString(e));
+  return NSA_OK;
+}
+
+// One tensor of a pooling launch: window means of x [slabs, T, D] into out [slabs, n_out, D] (pool_select.cu).
+struct PoolJob {
+  const void* x;
+  void* out;
+  int T, block, stride, n_out, slabs;
+  float dq;            // fp8 only: factor of the dequantisation
+  unsigned block0;     // filled in by the launcher
+};
+
 // ---------------------------------------------------------------- dtype traits
 template <typename T> struct Elem;
 template <> struct Elem<__nv_bfloat16> {

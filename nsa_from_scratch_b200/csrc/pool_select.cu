@@ -8,43 +8,73 @@
 namespace nsa {
 
 // ------------------------------------------------------------------ pooling
-// One thread produces 8 consecutive columns of one pooled row.
+// Window means of up to four tensors in one launch (a forward needs the block means of Q and K and the pooled K and
+// V).  One thread produces 8 consecutive columns of one pooled row.  Bound by HBM at long sequences and by the
+// latency of its dependent loads at short ones: the rows of a window are fetched 16 at a time before any is added, so
+// a 64-row window costs four memory round trips instead of one per row or two, and the four tensors share them.
+struct PoolJobs {
+  PoolJob j[4];
+  int n;
+};
+
 template <typename T, bool IN8>
-__global__ void __launch_bounds__(256) pool_mean_kernel(const void* __restrict__ xin, T* __restrict__ out, int Tlen, int D,
-                                                        int block, int stride, int n_out, float dq, int fmt) {
-  const int CH = D / 8;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_out * CH) return;
-  const int c = i / CH, ch = i % CH;
-  const size_t slab = (size_t)blockIdx.y * Tlen * D;
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  const int r0 = c * stride;
-  const int r1 = min(r0 + block, Tlen);
-  for (int r = r0; r < r1; ++r) {
-    if constexpr (IN8) {
-      const uint8_t* p = reinterpret_cast<const uint8_t*>(xin) + slab + (size_t)r * D + ch * 8;
-      uint2 raw = *reinterpret_cast<const uint2*>(p);
-      const uint8_t* b = reinterpret_cast<const uint8_t*>(&raw);
+__device__ __forceinline__ void pool_add(float (&acc)[8], const uint4& raw, float dq, int fmt) {
+  if constexpr (IN8) {
+    const uint32_t w[2] = {raw.x, raw.y};
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] += Elem<T>::to_f(Elem<T>::from_f(fp8_to_f(b[e], fmt) * dq));
-    } else {
-      const T* p = reinterpret_cast<const T*>(xin) + slab + (size_t)r * D + ch * 8;
-      uint4 raw = *reinterpret_cast<const uint4*>(p);
-      const uint32_t* w = reinterpret_cast<const uint32_t*>(&raw);
+    for (int e = 0; e < 8; ++e)
+      acc[e] += Elem<T>::to_f(Elem<T>::from_f(fp8_to_f((uint8_t)(w[e >> 2] >> ((e & 3) * 8)), fmt) * dq));
+  } else {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float2 f = Elem<T>::unpack(w[e]);
-        acc[2 * e] += f.x;
-        acc[2 * e + 1] += f.y;
-      }
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = Elem<T>::unpack(w[e]);
+      acc[2 * e] += f.x;
+      acc[2 * e + 1] += f.y;
     }
   }
-  const float inv_n = (float)block;
+}
+
+template <typename T, bool IN8>
+__global__ void __launch_bounds__(128) pool_mean_kernel(const __grid_constant__ PoolJobs p, int D, int fmt) {
+  constexpr int U = 16;
+  grid_dep_wait();
+  int k = 0;
+#pragma unroll
+  for (int e = 1; e < 4; ++e)
+    if (e < p.n && blockIdx.x >= p.j[e].block0) k = e;
+  const PoolJob& jb = p.j[k];
+  const unsigned CH = D / 8;
+  const unsigned per_slab = (unsigned)jb.n_out * CH;
+  const unsigned i = (blockIdx.x - jb.block0) * 128u + threadIdx.x;
+  if (i >= per_slab * (unsigned)jb.slabs) return;
+  const unsigned slab = i / per_slab, in = i % per_slab;
+  const int c = (int)(in / CH), ch = (int)(in % CH);
+  constexpr int ISZ = IN8 ? 1 : 2;
+  const int r0 = c * jb.stride;
+  const int r1 = min(r0 + jb.block, jb.T);
+  const unsigned char* src = reinterpret_cast<const unsigned char*>(jb.x) + ((size_t)slab * jb.T * D + ch * 8) * ISZ;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  auto row = [&](int r) {
+    const unsigned char* q = src + (size_t)r * D * ISZ;
+    if constexpr (IN8) { const uint2 v = *reinterpret_cast<const uint2*>(q); return make_uint4(v.x, v.y, 0u, 0u); }
+    else return *reinterpret_cast<const uint4*>(q);
+  };
+  int r = r0;
+  for (; r + U <= r1; r += U) {
+    uint4 raw[U];
+#pragma unroll
+    for (int e = 0; e < U; ++e) raw[e] = row(r + e);
+#pragma unroll
+    for (int e = 0; e < U; ++e) pool_add<T, IN8>(acc, raw[e], jb.dq, fmt);
+  }
+  for (; r < r1; ++r) pool_add<T, IN8>(acc, row(r), jb.dq, fmt);
+  grid_dep_launch();
+  const float inv_n = (float)jb.block;
   uint32_t w[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) w[e] = Elem<T>::pack(__fdiv_rn(acc[2 * e], inv_n), __fdiv_rn(acc[2 * e + 1], inv_n));
-  T* q = out + ((size_t)blockIdx.y * n_out + c) * D + ch * 8;
-  *reinterpret_cast<uint4*>(q) = make_uint4(w[0], w[1], w[2], w[3]);
+  *reinterpret_cast<uint4*>(reinterpret_cast<T*>(jb.out) + ((size_t)slab * jb.n_out + c) * D + ch * 8) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 // Learned pooling: out[c, d] = sum_s x[c*stride + s, d] * w[s, d] over the `block` rows of the window (rows past the
@@ -97,23 +127,44 @@ int pool_weighted(const void* x, const float* w, void* out, int B, int H, int T,
   return launch_status("pool_weighted");
 }
 
+static int n_windows(int T, int block, int stride) {
+  return stride == block ? (T + block - 1) / block : (T >= block ? (T - block) / stride + 1 : 0);
+}
+
+// Jobs of one element type and one D; empty ones are dropped.
+int pool_mean_multi(const PoolJob* jobs, int n_jobs, int D, int dtype, cudaStream_t st) {
+  NSA_REQUIRE(D % 8 == 0 && D > 0, NSA_ERR_ARG, "pool: D %d must be a positive multiple of 8", D);
+  PoolJobs p;
+  p.n = 0;
+  long long blocks = 0;
+  for (int k = 0; k < n_jobs; ++k) {
+    const PoolJob& jb = jobs[k];
+    NSA_REQUIRE(jb.block > 0 && jb.stride > 0 && jb.stride <= jb.block, NSA_ERR_ARG, "pool: need 0 < stride <= block (%d, %d)", jb.stride, jb.block);
+    NSA_REQUIRE(jb.n_out == n_windows(jb.T, jb.block, jb.stride), NSA_ERR_ARG, "pool: n_out %d, expected %d", jb.n_out,
+                n_windows(jb.T, jb.block, jb.stride));
+    if (jb.n_out == 0 || jb.slabs == 0) continue;
+    NSA_REQUIRE((long long)jb.slabs <= 65535, NSA_ERR_ARG, "pool: B*H %lld too large", (long long)jb.slabs);
+    const long long threads = (long long)jb.slabs * jb.n_out * (D / 8);
+    NSA_REQUIRE(threads < (1LL << 31), NSA_ERR_ARG, "pool: %lld results do not fit a launch", threads);
+    p.j[p.n] = jb;
+    p.j[p.n].block0 = (unsigned)blocks;
+    ++p.n;
+    blocks += (threads + 127) / 128;
+  }
+  if (p.n == 0) return NSA_OK;
+  switch (dtype) {
+    case NSA_BF16: return launch_pdl("pool_mean", pool_mean_kernel<__nv_bfloat16, false>, dim3((unsigned)blocks), 128, 0, st, p, D, 0);
+    case NSA_FP16: return launch_pdl("pool_mean", pool_mean_kernel<__half, false>, dim3((unsigned)blocks), 128, 0, st, p, D, 0);
+    case NSA_FP8_E4M3:
+    case NSA_FP8_E5M2: return launch_pdl("pool_mean", pool_mean_kernel<__nv_bfloat16, true>, dim3((unsigned)blocks), 128, 0, st, p, D, dtype);
+  }
+  return fail(NSA_ERR_UNSUPPORTED, "pool: dtype %d", dtype);
+}
+
 int pool_mean(const void* x, void* out, int B, int H, int T, int D, int block, int stride, int n_out, int dtype,
               float dq, cudaStream_t st) {
-  NSA_REQUIRE(D % 8 == 0 && D > 0, NSA_ERR_ARG, "pool: D %d must be a positive multiple of 8", D);
-  NSA_REQUIRE(block > 0 && stride > 0 && stride <= block, NSA_ERR_ARG, "pool: need 0 < stride <= block (%d, %d)", stride, block);
-  int expect = stride == block ? (T + block - 1) / block : (T >= block ? (T - block) / stride + 1 : 0);
-  NSA_REQUIRE(n_out == expect, NSA_ERR_ARG, "pool: n_out %d, expected %d", n_out, expect);
-  if (n_out == 0 || B * H == 0) return NSA_OK;
-  NSA_REQUIRE((long long)B * H <= 65535, NSA_ERR_ARG, "pool: B*H %lld too large", (long long)B * H);
-  dim3 grid((unsigned)(((long long)n_out * (D / 8) + 255) / 256), (unsigned)(B * H));
-  switch (dtype) {
-    case NSA_BF16: pool_mean_kernel<__nv_bfloat16, false><<<grid, 256, 0, st>>>(x, (__nv_bfloat16*)out, T, D, block, stride, n_out, 1.f, 0); break;
-    case NSA_FP16: pool_mean_kernel<__half, false><<<grid, 256, 0, st>>>(x, (__half*)out, T, D, block, stride, n_out, 1.f, 0); break;
-    case NSA_FP8_E4M3:
-    case NSA_FP8_E5M2: pool_mean_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(x, (__nv_bfloat16*)out, T, D, block, stride, n_out, dq, dtype); break;
-    default: return fail(NSA_ERR_UNSUPPORTED, "pool: dtype %d", dtype);
-  }
-  return launch_status("pool_mean");
+  const PoolJob jb = {x, out, T, block, stride, n_out, B * H, dq, 0u};
+  return pool_mean_multi(&jb, 1, D, dtype, st);
 }
 
 // ------------------------------------------------------------------ KV-cache append
@@ -422,6 +473,7 @@ __global__ void __launch_bounds__(256) select_blocks_kernel(const T* __restrict_
                                                             int force_first, int force_local, int R,
                                                             const int32_t* __restrict__ dyn_len) {
   constexpr int KT = 64;
+  grid_dep_wait();
   // key length in device memory (decoding under a captured graph): the padded-length offset of the block grid
   if (dyn_len != nullptr) offset = (*dyn_len + bn - 1) / bn * bn - ((nq * bm + bm - 1) / bm) * bm;
   constexpr int PITCH = D + 8;     // 16-bit elements; 16-byte aligned rows, 17-chunk stride -> conflict-free 128-bit reads
@@ -542,17 +594,16 @@ static int select_launch(const void* Qb, const void* Kb, int32_t* idx, int B, in
   {                                                                                                     \
     auto fn = select_blocks_kernel<T, DD>;                                                              \
     NSA_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));      \
-    fn<<<grid, 256, smem, st>>>((const T*)Qb, (const T*)Kb, idx, H, Hkv, Hi, nq, nk, k_out, bm, bn, offset, \
-                                causal, scale, ff, fl, R, dyn_len);                                     \
+    return launch_pdl("select_blocks", fn, grid, 256, smem, st, (const T*)Qb, (const T*)Kb, idx, H, Hkv, Hi, nq, nk, k_out, bm, bn, \
+                      offset, causal, scale, ff, fl, R, dyn_len);                                       \
   }
   switch (D) {
-    case 32: NSA_SEL(32) break;
-    case 64: NSA_SEL(64) break;
-    case 128: NSA_SEL(128) break;
-    default: return fail(NSA_ERR_UNSUPPORTED, "select: head dim %d not in {32,64,128}", D);
+    case 32: NSA_SEL(32)
+    case 64: NSA_SEL(64)
+    case 128: NSA_SEL(128)
   }
 #undef NSA_SEL
-  return launch_status("select_blocks");
+  return fail(NSA_ERR_UNSUPPORTED, "select: head dim %d not in {32,64,128}", D);
 }
 
 int select_blocks(const void* Qb, const void* Kb, int32_t* idx, int B, int H, int Hkv, int nq, int nk, int D, int top_k,

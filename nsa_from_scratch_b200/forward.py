@@ -2,9 +2,9 @@
 `nsa_forward` (:362-370), `_resolve_block_indices` (:321-324), `_block_scores_from_pooled`
 (:301-303) and the autograd Functions `_CompressedFn/_SelectedFn/_SlidingFn` (:123,143,263).
 
-Without autograd the whole forward is four launches: pool K/V, pool Q/K block means,
-score+top-k, and ONE fused kernel that runs the three branches per query tile and applies
-the gates in its epilogue (no branch output ever reaches HBM).  With autograd the branches
+Without autograd the whole forward is one library call and three launches: the window means of
+Q, K and V, score+top-k, and ONE fused kernel that runs the three branches per query tile and
+applies the gates in its epilogue (no branch output ever reaches HBM).  With autograd the branches
 run separately so that their outputs and log-sum-exps can be saved; every branch has a
 hand-written backward kernel (the reference differentiates its plain-torch functions for the
 compressed and sliding branches, nsa/triton/forward.py:133-140,273-298)."""
@@ -143,6 +143,13 @@ def _cfg(cfg, name, default):
     return default if v is None else v
 
 
+def _resolve_from_cfg(Q, K, cfg, scale, q_scale=1.0, k_scale=1.0):
+    return _resolve_block_indices(Q, K, block_size_m=cfg.block_size_m, block_size_n=cfg.block_size_n, top_k=cfg.top_k,
+                                  causal=cfg.causal, scale=scale, force_first=_cfg(cfg, "force_first", 0),
+                                  force_local=_cfg(cfg, "force_local", 0), q_scale=q_scale, k_scale=k_scale,
+                                  shared_per_group=bool(_cfg(cfg, "select_per_group", False)))
+
+
 def nsa_forward(Q: Tensor, K: Tensor, V: Tensor, cfg, *, gate_logits: Optional[Tensor] = None,
                 block_indices: Optional[Tensor] = None, pool_proj_k: Optional[Tensor] = None,
                 pool_proj_v: Optional[Tensor] = None) -> Tensor:
@@ -162,24 +169,20 @@ def nsa_forward(Q: Tensor, K: Tensor, V: Tensor, cfg, *, gate_logits: Optional[T
     if learned and (pool_proj_k is None or pool_proj_v is None):
         raise ValueError("nsa_forward: pool='learned' needs pool_proj_k and pool_proj_v ([block_size_c, D], nsa/reference.py:295-296)")
     stride_c = getattr(cfg, "stride_c", None)
-    ff, fl = _cfg(cfg, "force_first", 0), _cfg(cfg, "force_local", 0)
     if block_indices is None and _cfg(cfg, "scorer", "mean") == "compressed":
         from .scoring import forward_with_compressed_scorer, select_blocks_compressed
         if not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (Q, K, V, gate_logits))):
             return forward_with_compressed_scorer(Q, K, V, cfg, gate_logits)
         block_indices = select_blocks_compressed(Q, K, cfg)
-    elif block_indices is None:
-        if _cfg(cfg, "scorer", "mean") != "mean":
-            raise ValueError(f"unknown scorer: {cfg.scorer}")
-        block_indices = _resolve_block_indices(Q, K, block_size_m=cfg.block_size_m, block_size_n=cfg.block_size_n,
-                                               top_k=cfg.top_k, causal=cfg.causal, scale=float(scale),
-                                               force_first=ff, force_local=fl,
-                                               shared_per_group=bool(_cfg(cfg, "select_per_group", False)))
+    elif block_indices is None and _cfg(cfg, "scorer", "mean") != "mean":
+        raise ValueError(f"unknown scorer: {cfg.scorer}")
     needs_grad = torch.is_grad_enabled() and any(
         t is not None and t.requires_grad for t in (Q, K, V, gate_logits))
     if needs_grad and learned:
         raise NotImplementedError("nsa_forward: pool='learned' is forward-only here (no gradient kernels for the pooling weights)")
     if needs_grad:
+        if block_indices is None:
+            block_indices = _resolve_from_cfg(Q, K, cfg, float(scale))
         out_c = _CompressedFn.apply(Q, K, V, cfg.block_size_c, cfg.pool, cfg.causal, cfg.scale, stride_c)
         out_s = _SelectedFn.apply(Q, K, V, cfg.block_size_n, cfg.block_size_m, cfg.top_k, block_indices,
                                   cfg.causal, cfg.scale)
@@ -193,26 +196,36 @@ def nsa_forward(Q: Tensor, K: Tensor, V: Tensor, cfg, *, gate_logits: Optional[T
                           pool_proj=(pool_proj_k, pool_proj_v) if learned else None)
 
 
+def _gate_act(cfg) -> int:
+    if cfg.gate_activation == "sigmoid":
+        return L.GATE_SIGMOID
+    if cfg.gate_activation == "softmax":
+        return L.GATE_SOFTMAX
+    raise ValueError(f"unknown gate_activation: {cfg.gate_activation}")
+
+
 def _fused_forward(Q, K, V, cfg, scale, stride_c, gate_logits, block_indices, sq, sk, sv, engine=None,
                    token_major=False, pool_proj=None):
+    """block_indices None: chosen inside the call by block means."""
     bc = cfg.block_size_c
     stride = bc if stride_c is None else int(stride_c)
-    if pool_proj is not None:
-        Kc = ops.pool_learned(K, pool_proj[0], bc, stride)
-        Vc = ops.pool_learned(V, pool_proj[1], bc, stride)
-    else:
-        Kc = ops.pool_mean(K, bc, stride, dequant_scale=sk)
-        Vc = ops.pool_mean(V, bc, stride, dequant_scale=sv)
+    if pool_proj is None:
+        return ops.forward(
+            Q, K, V, causal=bool(cfg.causal), scale=scale, cmp_block=bc, cmp_stride=stride, bm=cfg.block_size_m, bn=cfg.block_size_n,
+            window=cfg.window_size, top_k=cfg.top_k, force_first=_cfg(cfg, "force_first", 0), force_local=_cfg(cfg, "force_local", 0),
+            per_group=bool(_cfg(cfg, "select_per_group", False)), idx=block_indices, gates=gate_logits, gate_act=_gate_act(cfg),
+            q_scale=sq, k_scale=sk, v_scale=sv, engine=engine, token_major=token_major)
+    if block_indices is None:
+        block_indices = _resolve_from_cfg(Q, K, cfg, scale, sq, sk)
+    Kc = ops.pool_learned(K, pool_proj[0], bc, stride)
+    Vc = ops.pool_learned(V, pool_proj[1], bc, stride)
     Tq, Tk = Q.shape[2], K.shape[2]
     Tk_pad = Kc.shape[2] * bc if stride == bc else Tk
-    if cfg.gate_activation not in ("sigmoid", "softmax"):
-        raise ValueError(f"unknown gate_activation: {cfg.gate_activation}")
     out, _ = ops.attention_fwd(
         Q, K, V, branches=L.BRANCH_COMPRESSED | L.BRANCH_SELECTED | L.BRANCH_SLIDING, fused=True,
         causal=bool(cfg.causal), scale=scale, Kc=Kc, Vc=Vc, cmp_block=bc, cmp_stride=stride, cmp_offset=Tk_pad - Tq,
         idx=block_indices, bm=cfg.block_size_m, bn=cfg.block_size_n, window=cfg.window_size, gates=gate_logits,
-        gate_act=L.GATE_SOFTMAX if cfg.gate_activation == "softmax" else L.GATE_SIGMOID,
-        q_scale=sq, k_scale=sk, v_scale=sv, engine=engine, token_major=token_major)
+        gate_act=_gate_act(cfg), q_scale=sq, k_scale=sk, v_scale=sv, engine=engine, token_major=token_major)
     return out
 
 
@@ -224,11 +237,6 @@ def nsa_forward_fp8(Q: Tensor, K: Tensor, V: Tensor, scale_q: float, scale_k: fl
     assert Q.dtype in (torch.float8_e4m3fn, torch.float8_e5m2) and K.dtype == Q.dtype and V.dtype == Q.dtype
     D = Q.shape[-1]
     scale = cfg.scale if cfg.scale is not None else 1.0 / (D ** 0.5)
-    if block_indices is None:
-        block_indices = _resolve_block_indices(
-            Q, K, block_size_m=cfg.block_size_m, block_size_n=cfg.block_size_n, top_k=cfg.top_k, causal=cfg.causal,
-            scale=float(scale), force_first=_cfg(cfg, "force_first", 0), force_local=_cfg(cfg, "force_local", 0),
-            q_scale=scale_q, k_scale=scale_k, shared_per_group=bool(_cfg(cfg, "select_per_group", False)))
     return _fused_forward(Q, K, V, cfg, float(scale), getattr(cfg, "stride_c", None), gate_logits, block_indices,
                           scale_q, scale_k, scale_v)
 

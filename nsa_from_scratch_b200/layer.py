@@ -20,7 +20,7 @@ import torch.nn as nn
 from torch import Tensor
 
 from . import ops
-from .forward import _cfg, _fused_forward, _resolve_block_indices, nsa_forward
+from .forward import _fused_forward, nsa_forward
 
 
 def rope_cache(seq_len: int, head_dim: int, base: float, device, dtype=torch.float32):
@@ -43,14 +43,10 @@ def nsa_attention_token_major(q: Tensor, k: Tensor, v: Tensor, cos: Optional[Ten
     kh = ops.rope_to_heads(k, cos, sin, dtype)
     vh = ops.rope_to_heads(v, None, None, dtype)
     scale = cfg.scale if cfg.scale is not None else 1.0 / (D ** 0.5)
-    idx = _resolve_block_indices(qh, kh, block_size_m=cfg.block_size_m, block_size_n=cfg.block_size_n, top_k=cfg.top_k,
-                                 causal=cfg.causal, scale=float(scale), force_first=_cfg(cfg, "force_first", 0),
-                                 force_local=_cfg(cfg, "force_local", 0),
-                                 shared_per_group=bool(_cfg(cfg, "select_per_group", False)))
     learned = getattr(cfg, "pool", "mean") == "learned"
     if learned and (pool_proj_k is None or pool_proj_v is None):
         raise ValueError("pool='learned' needs pool_proj_k and pool_proj_v")
-    out = _fused_forward(qh, kh, vh, cfg, float(scale), getattr(cfg, "stride_c", None), gate_logits, idx, 1.0, 1.0, 1.0,
+    out = _fused_forward(qh, kh, vh, cfg, float(scale), getattr(cfg, "stride_c", None), gate_logits, None, 1.0, 1.0, 1.0,
                          token_major=True, pool_proj=(pool_proj_k, pool_proj_v) if learned else None)
     return out.view(B, T, H * D)
 

@@ -99,7 +99,7 @@ def pool_mean(x: Tensor, block: int, stride: Optional[int] = None, dequant_scale
     n = n_pooled(T, block, stride)
     x = _dense(x, "x")
     out = torch.empty((B, H, n, D), device=x.device, dtype=torch.bfloat16 if x.dtype in _8 else x.dtype)
-    with torch.cuda.device(x.device):
+    with L.on_device(x):
         L.check(L.load().nsa_pool_mean(x.data_ptr(), out.data_ptr(), B, H, T, D, block, stride, n,
                                        L.dtype_code(x.dtype), float(dequant_scale), L.stream_ptr()), "nsa_pool_mean")
     return out
@@ -116,7 +116,7 @@ def pool_learned(x: Tensor, w: Tensor, block: int, stride: Optional[int] = None)
     x = _dense(x, "x")
     w = w.detach().to(torch.float32).contiguous()
     out = torch.empty((B, H, n, D), device=x.device, dtype=x.dtype)
-    with torch.cuda.device(x.device):
+    with L.on_device(x):
         L.check(L.load().nsa_pool_learned(x.data_ptr(), w.data_ptr(), out.data_ptr(), B, H, T, D, block, stride, n,
                                           L.dtype_code(x.dtype), L.stream_ptr()), "nsa_pool_learned")
     return out
@@ -130,7 +130,7 @@ def select_blocks_from_means(Qb: Tensor, Kb: Tensor, *, top_k: int, bm: int, bn:
     Hkv, nk = Kb.shape[1], Kb.shape[2]
     k_out = min(top_k, nk)
     idx = torch.empty((B, Hkv if shared_per_group else H, nq, k_out), device=Qb.device, dtype=torch.int32)
-    with torch.cuda.device(Qb.device):
+    with L.on_device(Qb):
         L.check(L.load().nsa_select_blocks(Qb.data_ptr(), Kb.data_ptr(), idx.data_ptr(), B, H, Hkv, nq, nk, D, top_k,
                                            bm, bn, offset, int(causal), float(scale), force_first, force_local,
                                            int(shared_per_group), L.dtype_code(Qb.dtype), L.stream_ptr()), "nsa_select_blocks")
@@ -154,13 +154,13 @@ def cmp_block_scores(Q: Tensor, Kc: Tensor, lse: Tensor, *, nk: int, cmp_block: 
     if (_ENGINE != L.ENGINE_GENERIC and D in (64, 128) and (bn + cmp_block) // cmp_stride + 1 <= 64 and fixed <= 225 * 1024
             and bn % cmp_stride == 0 and cmp_block % cmp_stride == 0):
         scratch = torch.empty((B, H, nq, nk), device=Q.device, dtype=torch.float32)
-        with torch.cuda.device(Q.device):
+        with L.on_device(Q):
             L.check(L.load().nsa_cmp_block_scores_tc(Q.data_ptr(), Kc.data_ptr(), lse.data_ptr(), scores.data_ptr(), scratch.data_ptr(),
                                                      B, H, Hkv, Tq, Nc, D, nk, cmp_block, cmp_stride, cmp_offset, bn, sel_offset,
                                                      int(causal), float(scale), force_first, force_local, int(shared_per_group),
                                                      L.dtype_code(Q.dtype), L.stream_ptr()), "nsa_cmp_block_scores_tc")
         return scores
-    with torch.cuda.device(Q.device):
+    with L.on_device(Q):
         L.check(L.load().nsa_cmp_block_scores(Q.data_ptr(), Kc.data_ptr(), lse.data_ptr(), scores.data_ptr(), B, H, Hkv, Tq, Nc, D,
                                               nk, cmp_block, cmp_stride, cmp_offset, bn, sel_offset, int(causal), float(scale),
                                               force_first, force_local, int(shared_per_group), L.dtype_code(Q.dtype),
@@ -173,7 +173,7 @@ def topk_from_scores(scores: Tensor, *, top_k: int, bm: int, bn: int, offset: in
     B, H, nq, nk = scores.shape
     scores = scores.float().contiguous()
     idx = torch.empty((B, H, nq, min(top_k, nk)), device=scores.device, dtype=torch.int32)
-    with torch.cuda.device(scores.device):
+    with L.on_device(scores):
         L.check(L.load().nsa_topk_from_scores(scores.data_ptr(), idx.data_ptr(), B * H, nq, nk, top_k, bm, bn, offset,
                                               int(causal), L.stream_ptr()), "nsa_topk_from_scores")
     return idx
@@ -269,9 +269,76 @@ def attention_fwd(
             raise ValueError("dyn_len must be a one-element int32 CUDA tensor")
         keep.append(dyn_len)
         a.dyn_len = dyn_len.data_ptr()
-    with torch.cuda.device(Q.device):
+    with L.on_device(Q):
         L.check(L.load().nsa_attention_fwd(C.byref(a), L.stream_ptr()), "nsa_attention_fwd")
     return out, lse
+
+
+# nsa_forward_args of the problems seen so far, pointers left out: (bytes of the struct, workspace bytes)
+_forward_plans: dict = {}
+
+
+def forward(Q: Tensor, K: Tensor, V: Tensor, *, causal: bool, scale: float, cmp_block: int, cmp_stride: int, bm: int, bn: int, window: int,
+            top_k: int, force_first: int = 0, force_local: int = 0, per_group: bool = False, idx: Optional[Tensor] = None,
+            gates: Optional[Tensor] = None, gate_act: int = L.GATE_SIGMOID, q_scale: float = 1.0, k_scale: float = 1.0,
+            v_scale: float = 1.0, engine: Optional[int] = None, token_major: bool = False) -> Tensor:
+    """The whole forward (window means, selection unless `idx` is given, the fused launch) as one library call."""
+    _need_cuda(Q, K, V)
+    q_shape, k_shape, dtype = Q.shape, K.shape, Q.dtype
+    B, H, Tq, D = q_shape
+    Q, K, V = _dense(Q, "Q"), _dense(K, "K"), _dense(V, "V")
+    if idx is not None:
+        idx = idx.to(torch.int32).contiguous()
+    if gates is not None:
+        gates = _dense(gates, "gates")
+    eng = _ENGINE if engine is None else engine
+    key = (q_shape, k_shape, dtype, causal, scale, cmp_block, cmp_stride, bm, bn, window, top_k, force_first, force_local, per_group,
+           None if idx is None else idx.shape, None if gates is None else gates.dtype, gate_act, q_scale, k_scale, v_scale, eng,
+           token_major)
+    plan = _forward_plans.get(key)
+    if V.shape != k_shape or V.dtype != dtype or K.dtype != dtype:
+        if V.shape != k_shape:
+            raise ValueError(f"K/V shapes {tuple(k_shape)}/{tuple(V.shape)} do not match Q {tuple(q_shape)}")
+        raise TypeError("Q, K, V must share a dtype")
+    if gates is not None and gates.shape != ((B, Tq, H, 3) if token_major else (B, H, Tq, 3)):
+        raise ValueError(f"gate_logits shape {tuple(gates.shape)} != {(B, Tq, H, 3) if token_major else (B, H, Tq, 3)}")
+    if plan is None:
+        Hkv, Tk = k_shape[1], k_shape[2]
+        if k_shape != (B, Hkv, Tk, D):
+            raise ValueError(f"K/V shapes {tuple(k_shape)}/{tuple(V.shape)} do not match Q {tuple(q_shape)}")
+        if H % Hkv:
+            raise ValueError(f"query heads {H} not a multiple of KV heads {Hkv}")
+        a = L.ForwardArgs()
+        a.B, a.H, a.Hkv, a.Tq, a.Tk, a.D = B, H, Hkv, Tq, Tk, D
+        a.top_k, a.force_first, a.force_local, a.per_group = int(top_k), int(force_first), int(force_local), int(per_group)
+        if idx is not None:
+            nq = (Tq + bm - 1) // bm
+            if idx.dim() != 4 or idx.shape[0] != B or idx.shape[1] not in (H, Hkv) or idx.shape[2] != nq:
+                raise ValueError(f"block_indices shape {tuple(idx.shape)} does not match (B={B}, H={H}|{Hkv}, nq={nq}, k)")
+            a.has_idx, a.Hi, a.top_k = 1, idx.shape[1], idx.shape[3]
+        a.cmp_block, a.cmp_stride, a.bm, a.bn, a.window, a.causal = cmp_block, cmp_stride, bm, bn, int(window), int(causal)
+        a.gate_act, a.q_dtype, a.engine = gate_act, L.dtype_code(dtype), eng
+        a.gate_dtype = 0 if gates is None else L.dtype_code(gates.dtype)
+        a.io_layout = (L.IO_OUT_BTHD | L.IO_GATES_BTHD) if token_major else 0
+        a.scale, a.q_scale, a.k_scale, a.v_scale = float(scale), float(q_scale), float(k_scale), float(v_scale)
+        need = int(L.load().nsa_forward_ws_bytes(C.byref(a)))
+        if need < 0:
+            L.check(need, "nsa_forward")
+        if len(_forward_plans) >= 256:       # a program meets few shapes; one that meets many starts over
+            _forward_plans.clear()
+        plan = _forward_plans[key] = (bytes(a), need)
+    a = L.ForwardArgs.from_buffer_copy(plan[0])
+    dev = Q.device
+    out = torch.empty((B, Tq, H, D) if token_major else q_shape, device=dev, dtype=torch.bfloat16 if dtype in _8 else dtype)
+    ws = torch.empty(plan[1], device=dev, dtype=torch.uint8)
+    a.Q, a.K, a.V, a.out, a.ws, a.ws_bytes = Q.data_ptr(), K.data_ptr(), V.data_ptr(), out.data_ptr(), ws.data_ptr(), plan[1]
+    if gates is not None:
+        a.gates = gates.data_ptr()
+    if idx is not None:
+        a.idx = idx.data_ptr()
+    with L.on_device(Q):
+        L.check(L.load().nsa_forward(C.byref(a), L.stream_ptr()), "nsa_forward")
+    return out
 
 
 def bwd_delta(dO: Tensor, O: Tensor) -> Tensor:
@@ -279,7 +346,7 @@ def bwd_delta(dO: Tensor, O: Tensor) -> Tensor:
     dO, O = _dense(dO, "dO"), _dense(O, "O")
     D = dO.shape[-1]
     delta = torch.empty(dO.shape[:-1], device=dO.device, dtype=torch.float32)
-    with torch.cuda.device(dO.device):
+    with L.on_device(dO):
         L.check(L.load().nsa_bwd_delta(dO.data_ptr(), O.data_ptr(), delta.data_ptr(), delta.numel(), D,
                                        L.dtype_code(dO.dtype), L.stream_ptr()), "nsa_bwd_delta")
     return delta
@@ -318,7 +385,7 @@ def attention_bwd(dO: Tensor, Q: Tensor, K: Tensor, V: Tensor, lse: Tensor, delt
     else:
         a.Nc, a.cmp_block, a.cmp_stride, a.cmp_offset = rows, cmp_block, cmp_stride, cmp_offset
     a.engine = _BWD_ENGINE
-    with torch.cuda.device(Q.device):
+    with L.on_device(Q):
         lib = L.load()
         scratch = None
         if _BWD_ENGINE != L.ENGINE_GENERIC:
@@ -343,7 +410,7 @@ def pool_mean_bwd(dxc: Tensor, T: int, block: int, stride: int) -> Tensor:
     B, H, n, D = dxc.shape
     dxc = _dense(dxc, "dxc")
     dx = torch.zeros((B, H, T, D), device=dxc.device, dtype=torch.float32)
-    with torch.cuda.device(dxc.device):
+    with L.on_device(dxc):
         L.check(L.load().nsa_pool_mean_bwd(dxc.data_ptr(), dx.data_ptr(), B, H, T, D, block, stride, n, L.stream_ptr()),
                 "nsa_pool_mean_bwd")
     return dx
@@ -353,7 +420,7 @@ def cast_from_f32(x: Tensor, dtype: torch.dtype) -> Tensor:
     _need_cuda(x)
     x = _dense(x, "x")
     out = torch.empty(x.shape, device=x.device, dtype=dtype)
-    with torch.cuda.device(x.device):
+    with L.on_device(x):
         L.check(L.load().nsa_cast_from_f32(x.data_ptr(), out.data_ptr(), x.numel(), L.dtype_code(dtype), L.stream_ptr()),
                 "nsa_cast_from_f32")
     return out
@@ -376,7 +443,7 @@ def rope_to_heads(x: Tensor, cos: Optional[Tensor], sin: Optional[Tensor], dtype
         cos, sin = _dense(cos, "cos"), _dense(sin, "sin")
         cs_code = L.dtype_code(cos.dtype)
     y = torch.empty((B, H, T, D), device=x.device, dtype=dtype)
-    with torch.cuda.device(x.device):
+    with L.on_device(x):
         L.check(L.load().nsa_rope_to_heads(x.data_ptr(), y.data_ptr(), L.ptr(cos), L.ptr(sin), B, T, H, D,
                                            L.dtype_code(x.dtype), cs_code, L.dtype_code(dtype), L.stream_ptr()),
                 "nsa_rope_to_heads")
@@ -418,7 +485,7 @@ def combine(out_c: Tensor, out_s: Tensor, out_w: Tensor, gate_logits: Tensor, ac
         raise ValueError(f"gate_logits shape {tuple(gate_logits.shape)} != {(B, H, Tq, 3)}")
     out_c, out_s, out_w, g = _dense(out_c, "out_c"), _dense(out_s, "out_s"), _dense(out_w, "out_w"), _dense(gate_logits, "gate_logits")
     out = torch.empty((B, H, Tq, D), device=out_c.device, dtype=torch.float32 if g.dtype == torch.float32 else out_c.dtype)
-    with torch.cuda.device(out_c.device):
+    with L.on_device(out_c):
         L.check(L.load().nsa_combine(out_c.data_ptr(), out_s.data_ptr(), out_w.data_ptr(), g.data_ptr(), out.data_ptr(),
                                      B * H * Tq, D, L.GATE_SOFTMAX if activation == "softmax" else L.GATE_SIGMOID,
                                      L.dtype_code(out_c.dtype), L.dtype_code(g.dtype), L.stream_ptr()), "nsa_combine")
@@ -429,7 +496,7 @@ def fp8_absmax(x: Tensor) -> Tensor:
     _need_cuda(x)
     x = _dense(x, "x")
     out = torch.zeros(1, device=x.device, dtype=torch.float32)
-    with torch.cuda.device(x.device):
+    with L.on_device(x):
         L.check(L.load().nsa_fp8_absmax(x.data_ptr(), x.numel(), L.dtype_code(x.dtype), out.data_ptr(), L.stream_ptr()),
                 "nsa_fp8_absmax")
     return out
@@ -440,7 +507,7 @@ def fp8_dequantize(x8: Tensor, scale: float) -> Tensor:
     _need_cuda(x8)
     x8 = _dense(x8, "x8")
     out = torch.empty(x8.shape, device=x8.device, dtype=torch.bfloat16)
-    with torch.cuda.device(x8.device):
+    with L.on_device(x8):
         L.check(L.load().nsa_fp8_dequantize(x8.data_ptr(), out.data_ptr(), x8.numel(), L.dtype_code(x8.dtype), float(scale),
                                             L.stream_ptr()), "nsa_fp8_dequantize")
     return out
@@ -450,7 +517,7 @@ def fp8_quantize(x: Tensor, fmt: torch.dtype, scale: float) -> Tensor:
     _need_cuda(x)
     x = _dense(x, "x")
     out = torch.empty(x.shape, device=x.device, dtype=torch.uint8)
-    with torch.cuda.device(x.device):
+    with L.on_device(x):
         L.check(L.load().nsa_fp8_quantize(x.data_ptr(), out.data_ptr(), x.numel(), L.dtype_code(x.dtype),
                                           L.dtype_code(fmt), float(scale), L.stream_ptr()), "nsa_fp8_quantize")
     return out.view(fmt)

@@ -1,0 +1,46 @@
+"""The forward as one library call: its window means at the edges of their load batches, and the whole call against
+the same steps taken one by one."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def nsa():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import nsa_from_scratch_b200 as m
+    return m
+
+
+@pytest.mark.parametrize("block,stride", [(1, 1), (15, 15), (16, 16), (17, 17), (33, 11), (64, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_window_means_are_row_order_sums(nsa, block, stride, dtype):
+    """fp32 sum in row order, one exact division, one rounding: bit-equal to the same steps in torch."""
+    from nsa_from_scratch_b200 import ops
+    T, D = 131, 64
+    x = torch.randn(2, 3, T, D, generator=torch.Generator().manual_seed(block)).to(dtype)
+    n = ops.n_pooled(T, block, stride)
+    want = torch.zeros(2, 3, n, D)
+    for s in range(block):
+        rows = torch.arange(n) * stride + s
+        want += torch.where((rows < T)[:, None], x[:, :, rows.clamp(max=T - 1)].float(), torch.zeros(()))
+    got = ops.pool_mean(x.cuda(), block, stride).cpu()
+    assert torch.equal(got, (want / block).to(dtype))
+
+
+@pytest.mark.parametrize("H,Hkv,T,Tq,D,group", [(4, 4, 64, 64, 64, False), (8, 2, 257, 257, 128, True), (4, 1, 300, 65, 64, True), (2, 2, 33, 33, 64, False)])
+def test_one_call_equals_the_steps(nsa, H, Hkv, T, Tq, D, group):
+    from nsa_from_scratch_b200 import _lib as L, ops
+    g = torch.Generator().manual_seed(3)
+    Q, K, V = (torch.randn(1, h, t, D, generator=g).to(torch.bfloat16).cuda() for h, t in ((H, Tq), (Hkv, T), (Hkv, T)))
+    gates = torch.randn(1, H, Tq, 3, generator=g).cuda()
+    cfg = nsa.NSAConfig(block_size_c=32, stride_c=16, top_k=3, window_size=70, force_first=1, force_local=1, select_per_group=group)
+    idx = nsa._resolve_block_indices(Q, K, block_size_m=64, block_size_n=64, top_k=3, causal=True, scale=D ** -0.5, force_first=1,
+                                     force_local=1, shared_per_group=group)
+    want, _ = ops.attention_fwd(Q, K, V, branches=7, fused=True, causal=True, scale=D ** -0.5, Kc=ops.pool_mean(K, 32, 16),
+                                Vc=ops.pool_mean(V, 32, 16), cmp_block=32, cmp_stride=16, cmp_offset=T - Tq, idx=idx, window=70,
+                                gates=gates, gate_act=L.GATE_SIGMOID)
+    assert torch.equal(nsa.nsa_forward(Q, K, V, cfg, gate_logits=gates), want)
+    assert torch.equal(nsa.nsa_forward(Q, K, V, cfg, gate_logits=gates, block_indices=idx), want)
