@@ -222,6 +222,20 @@ typedef struct nsa_forward_args {
 int64_t nsa_forward_ws_bytes(const nsa_forward_args* args);
 int nsa_forward(const nsa_forward_args* args, nsa_stream_t stream);
 
+/* The same forward for training (16-bit storage, io_layout 0): the branches run separately so that their outputs and
+ * log-sum-exps can be kept, then the gated combine.  branch_out [3,B,H,Tq,D] (Q's type), branch_lse [3,B,H,Tq] fp32,
+ * idx [B,Hi,nq,min(top_k,nk)] (written unless args->has_idx), Kc/Vc [B,Hkv,Nc,D]; out in Q's type.
+ * Replaces: the autograd route of nsa_forward, nsa/triton/forward.py:123-298. */
+int nsa_forward_train(const nsa_forward_args* args, void* branch_out, float* branch_lse, int32_t* idx, void* Kc, void* Vc, nsa_stream_t stream);
+
+/* Gradients of that forward: dQ, dK, dV in Q's type, dgates [B,H,Tq,3] in the gate logits' type (NULL: not wanted).
+ * args as in the forward, with ws / ws_bytes for this call: nsa_backward_ws_bytes(args) bytes, 256-byte aligned; 0
+ * means that the shape is not taken (D in {64,128}, 64-token blocks, at most 64 listed blocks, at least one pooled token).
+ * dQ repeats bit for bit; dK and dV are summed with fp32 reductions whose order is not fixed. */
+int64_t nsa_backward_ws_bytes(const nsa_forward_args* args);
+int nsa_backward(const nsa_forward_args* args, const void* dO, const void* branch_out, const float* branch_lse, const int32_t* idx,
+                 const void* Kc, const void* Vc, void* dQ, void* dK, void* dV, void* dgates, nsa_stream_t stream);
+
 /* Synchronises `stream`, then reports whether any kernel launched so far gave up on one of
  * its bounded device-side waits: NSA_OK, or NSA_ERR_DEVICE (and the condition is cleared).
  * No counterpart in the reference (its kernels have no device-side waits). */

@@ -102,6 +102,9 @@ PROTOTYPES = {
     "nsa_attention_fwd": (_i, [C.POINTER(FwdArgs), _vp]),
     "nsa_forward_ws_bytes": (_i64, [C.POINTER(ForwardArgs)]),
     "nsa_forward": (_i, [C.POINTER(ForwardArgs), _vp]),
+    "nsa_forward_train": (_i, [C.POINTER(ForwardArgs)] + [_vp] * 6),
+    "nsa_backward_ws_bytes": (_i64, [C.POINTER(ForwardArgs)]),
+    "nsa_backward": (_i, [C.POINTER(ForwardArgs)] + [_vp] * 11),
     "nsa_device_status": (_i, [_vp]),
     "nsa_debug_set_device_status": (_i, [_i, _i]),
     "nsa_compressed_attention_static": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp]),

@@ -30,12 +30,13 @@ int tc5_take_status(cudaStream_t, int*);
 int attention_bwd(const nsa_bwd_args&, cudaStream_t);
 bool attention_bwd_tc5_supports(const nsa_bwd_args&);
 long long attention_bwd_tc5_scratch_bytes(const nsa_bwd_args&);
-int attention_bwd_tc5(const nsa_bwd_args&, void*, long long, cudaStream_t);
+int attention_bwd_tc5(const nsa_bwd_args&, void*, long long, bool, cudaStream_t);
+int bst_take_status(int*);
 int bw5_take_status(int*);
 int tc5_set_status(int);
 int bw5_set_status(int);
 int pool_mean_bwd(const float*, float*, int, int, int, int, int, int, int, cudaStream_t);
-int combine(const void*, const void*, const void*, const void*, void*, long long, int, int, int, int, cudaStream_t);
+int combine(const void*, const void*, const void*, const void*, void*, long long, int, int, int, int, int, cudaStream_t);
 int fp8_absmax(const void*, long long, int, float*, cudaStream_t);
 int fp8_quantize(const void*, void*, long long, int, int, float, cudaStream_t);
 int fp8_dequantize(const void*, void*, long long, int, float, cudaStream_t);
@@ -210,6 +211,9 @@ int nsa_device_status(nsa_stream_t stream) {
   int v3 = 0;
   if ((rc = bw5_take_status(&v3)) != NSA_OK) return rc;
   if (v == 0 && v3 != 0) v = 200 + v3;
+  int v4 = 0;
+  if ((rc = bst_take_status(&v4)) != NSA_OK) return rc;
+  if (v == 0 && v4 != 0) v = 300 + v4;
   if (v != 0) return fail(NSA_ERR_DEVICE, "a kernel gave up waiting on barrier %d (bounded wait expired)", v - 1);
   return NSA_OK;
 }
@@ -275,9 +279,9 @@ int nsa_attention_bwd(const nsa_bwd_args* a, nsa_stream_t stream) {
   const bool tc5 = attention_bwd_tc5_supports(b);
   if (b.engine == NSA_ENGINE_TCGEN05) {
     NSA_REQUIRE(tc5, NSA_ERR_UNSUPPORTED, "attention backward: the tcgen05 engine does not take this shape or branch");
-    return attention_bwd_tc5(b, b.scratch, b.scratch_bytes, (cudaStream_t)stream);
+    return attention_bwd_tc5(b, b.scratch, b.scratch_bytes, false, (cudaStream_t)stream);
   }
-  if (b.engine == NSA_ENGINE_AUTO && tc5 && b.scratch != nullptr) return attention_bwd_tc5(b, b.scratch, b.scratch_bytes, (cudaStream_t)stream);
+  if (b.engine == NSA_ENGINE_AUTO && tc5 && b.scratch != nullptr) return attention_bwd_tc5(b, b.scratch, b.scratch_bytes, false, (cudaStream_t)stream);
   return attention_bwd(b, (cudaStream_t)stream);
 }
 
@@ -331,7 +335,8 @@ int launch_selected_attn_bwd(const void* Q, const void* K, const void* V, const 
 int nsa_combine(const void* out_c, const void* out_s, const void* out_w, const void* gates, void* out, int64_t rows,
                 int D, int activation, int dtype, int gate_dtype, nsa_stream_t stream) {
   NSA_REQUIRE(out_c && out_s && out_w && gates && out, NSA_ERR_ARG, "combine: NULL pointer");
-  return combine(out_c, out_s, out_w, gates, out, rows, D, activation, dtype, gate_dtype, (cudaStream_t)stream);
+  return combine(out_c, out_s, out_w, gates, out, rows, D, activation, dtype, gate_dtype, gate_dtype == NSA_FP32 ? NSA_FP32 : dtype,
+                 (cudaStream_t)stream);
 }
 
 int nsa_fp8_absmax(const void* x, int64_t n, int dtype, float* absmax, nsa_stream_t stream) {

@@ -807,7 +807,8 @@ static Bw5Plan bw5_plan(const nsa_bwd_args& a) {
 
 long long attention_bwd_tc5_scratch_bytes(const nsa_bwd_args& a) { return (long long)bw5_plan(a).total; }
 
-int attention_bwd_tc5(const nsa_bwd_args& a, void* scratch, long long scratch_bytes, cudaStream_t st) {
+// keys_only: dK and dV alone (the whole forward's backward forms dQ in its own pass over all branches)
+int attention_bwd_tc5(const nsa_bwd_args& a, void* scratch, long long scratch_bytes, bool keys_only, cudaStream_t st) {
   const Bw5Plan pl = bw5_plan(a);
   NSA_REQUIRE(scratch != nullptr && scratch_bytes >= (long long)pl.total, NSA_ERR_ARG,
               "selected backward (tcgen05): needs %lld bytes of scratch, %lld given", (long long)pl.total, scratch_bytes);
@@ -864,7 +865,7 @@ int attention_bwd_tc5(const nsa_bwd_args& a, void* scratch, long long scratch_by
     f0<<<grid0, BW5_THREADS, smem0, st>>>(p);                                                                     \
     bw5_reduce_kernel<DD><<<dim3((unsigned)pl.nkb, (unsigned)pl.owners), 256, 0, st>>>(partials, seginfo, a.dK_f, a.dV_f, pl.nkb, \
                                                                                        pl.capP, a.Tk);           \
-    f1<<<(unsigned)tiles1, BW5_THREADS, smem1, st>>>(p);                                                          \
+    if (!keys_only) f1<<<(unsigned)tiles1, BW5_THREADS, smem1, st>>>(p);                                          \
   }
   const int fmt = a.dtype == NSA_BF16 ? 1 : 0;
   if (a.D == 128 && fmt == 1) NSA_BW5_LAUNCH(128, 1)

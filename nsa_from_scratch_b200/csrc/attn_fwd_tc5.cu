@@ -1691,9 +1691,14 @@ int make_map(CUtensorMap* m, const void* ptr, long long slabs, long long rows, i
   cuuint64_t strides[2] = {(cuuint64_t)D * 2, (cuuint64_t)rows * D * 2};
   cuuint32_t box[3] = {64, 64, 1};
   cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(m, dtype == NSA_FP16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
+  auto encode = [&] { return enc(m, dtype == NSA_FP16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
                    const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {     // a thread that has not used the runtime yet (autograd's): bind the device's context to it
+    NSA_CUDA_OK(cudaFree(nullptr));
+    r = encode();
+  }
   NSA_REQUIRE(r == CUDA_SUCCESS, NSA_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
   return NSA_OK;
 }

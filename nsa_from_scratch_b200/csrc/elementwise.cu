@@ -32,13 +32,15 @@ template <typename T>
 __global__ void __launch_bounds__(256) combine16_kernel(const T* __restrict__ oc, const T* __restrict__ os,
                                                         const T* __restrict__ ow, const void* __restrict__ gates,
                                                         void* __restrict__ out, long long rows, int D, int act,
-                                                        int dt, int gdt) {
+                                                        int dt, int gdt, int odt) {
+  grid_dep_wait();
   const int CH = D / 8;
   const long long total = rows * CH;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / CH;
     const int ch = (int)(i % CH);
-    float x0 = load_any(gates, r * 3 + 0, gdt), x1 = load_any(gates, r * 3 + 1, gdt), x2 = load_any(gates, r * 3 + 2, gdt);
+    float x0 = 0.f, x1 = 0.f, x2 = 0.f;
+    if (gates != nullptr) { x0 = load_any(gates, r * 3 + 0, gdt); x1 = load_any(gates, r * 3 + 1, gdt); x2 = load_any(gates, r * 3 + 2, gdt); }
     float g0, g1, g2;
     if (act == NSA_GATE_SOFTMAX) {
       float mx = fmaxf(x0, fmaxf(x1, x2));
@@ -75,6 +77,11 @@ __global__ void __launch_bounds__(256) combine16_kernel(const T* __restrict__ oc
         o[2 * e] = (g0 * fa.x + g1 * fb.x) + g2 * fc.x;
         o[2 * e + 1] = (g0 * fa.y + g1 * fb.y) + g2 * fc.y;
       }
+      if (odt != NSA_FP32) {                               // fp32 gates, result rounded once to the branches' type
+        *reinterpret_cast<uint4*>(reinterpret_cast<T*>(out) + e0i) =
+            make_uint4(Elem<T>::pack(o[0], o[1]), Elem<T>::pack(o[2], o[3]), Elem<T>::pack(o[4], o[5]), Elem<T>::pack(o[6], o[7]));
+        continue;
+      }
       float4* q = reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + e0i);
       q[0] = make_float4(o[0], o[1], o[2], o[3]);
       q[1] = make_float4(o[4], o[5], o[6], o[7]);
@@ -83,7 +90,7 @@ __global__ void __launch_bounds__(256) combine16_kernel(const T* __restrict__ oc
 }
 
 int combine(const void* oc, const void* os, const void* ow, const void* gates, void* out, long long rows, int D,
-            int act, int dtype, int gate_dtype, cudaStream_t st) {
+            int act, int dtype, int gate_dtype, int out_dtype, cudaStream_t st) {
   NSA_REQUIRE(D > 0 && D % 8 == 0, NSA_ERR_ARG, "combine: D %d must be a multiple of 8", D);
   NSA_REQUIRE(act == NSA_GATE_SIGMOID || act == NSA_GATE_SOFTMAX, NSA_ERR_ARG, "combine: activation %d", act);
   NSA_REQUIRE(gate_dtype == dtype || gate_dtype == NSA_FP32, NSA_ERR_UNSUPPORTED,
@@ -91,14 +98,12 @@ int combine(const void* oc, const void* os, const void* ow, const void* gates, v
   if (rows == 0) return NSA_OK;
   int grid = grid_for(rows * (D / 8), 256);
   if (dtype == NSA_BF16)
-    combine16_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)oc, (const __nv_bfloat16*)os,
-                                                          (const __nv_bfloat16*)ow, gates, out, rows, D, act, dtype, gate_dtype);
-  else if (dtype == NSA_FP16)
-    combine16_kernel<__half><<<grid, 256, 0, st>>>((const __half*)oc, (const __half*)os, (const __half*)ow, gates, out,
-                                                   rows, D, act, dtype, gate_dtype);
-  else
-    return fail(NSA_ERR_UNSUPPORTED, "combine: dtype %d", dtype);
-  return launch_status("combine");
+    return launch_pdl("combine", combine16_kernel<__nv_bfloat16>, dim3(grid), 256, 0, st, (const __nv_bfloat16*)oc, (const __nv_bfloat16*)os,
+                      (const __nv_bfloat16*)ow, gates, out, rows, D, act, dtype, gate_dtype, out_dtype);
+  if (dtype == NSA_FP16)
+    return launch_pdl("combine", combine16_kernel<__half>, dim3(grid), 256, 0, st, (const __half*)oc, (const __half*)os, (const __half*)ow,
+                      gates, out, rows, D, act, dtype, gate_dtype, out_dtype);
+  return fail(NSA_ERR_UNSUPPORTED, "combine: dtype %d", dtype);
 }
 
 // ------------------------------------------------------------------ fp8 absmax / quantise

@@ -2,6 +2,8 @@
 // three-branch attention launch, in a workspace the caller provides.  A short forward is bound by the host and by
 // the gaps between its launches: issued from here the step costs three launches (six before: one per pooled tensor)
 // and one library call, and the small kernels follow each other through programmatic dependent launch.
+// The training forward keeps what the backward needs (the branch outputs and their log-sum-exps, the block lists, the
+// pooled keys and values); the backward is one call too (attn_bwd_stream.cu).
 #include "common.cuh"
 
 namespace nsa {
@@ -11,6 +13,10 @@ int select_blocks(const void*, const void*, int32_t*, int, int, int, int, int, i
                   int, int, int, const int32_t*, cudaStream_t);
 bool attention_fwd_tc5_supports(const nsa_fwd_args&);
 int fp8_dequantize(const void*, void*, long long, int, float, cudaStream_t);
+int combine(const void*, const void*, const void*, const void*, void*, long long, int, int, int, int, int, cudaStream_t);
+long long backward_ws_bytes(const nsa_forward_args&);
+int backward_stream(const nsa_forward_args&, const void*, const void*, const float*, const int32_t*, const void*, const void*, void*, void*, void*,
+                    void*, cudaStream_t);
 
 static bool fp8(int dt) { return dt == NSA_FP8_E4M3 || dt == NSA_FP8_E5M2; }
 
@@ -54,6 +60,22 @@ static int forward_plan(const nsa_forward_args& f, ForwardPlan& pl) {
   pl.o_v16 = o; if (pl.dequant) o = up(o + kv * f.Tk * row);
   pl.total = o < 256 ? 256 : o;
   return NSA_OK;
+}
+
+// Everything of the attention launch but the branches and what is written.
+static nsa_fwd_args attention_args(const nsa_forward_args& f, const ForwardPlan& pl, const void* K, const void* V, const void* Kc, const void* Vc,
+                                   const int32_t* idx) {
+  nsa_fwd_args a = {};
+  a.Q = f.Q; a.K = K; a.V = V; a.Kc = Kc; a.Vc = Vc; a.idx = idx;
+  a.B = f.B; a.H = f.H; a.Hkv = f.Hkv; a.Hi = pl.Hi; a.Tq = f.Tq; a.Tk = f.Tk; a.D = f.D; a.offset = f.Tk - f.Tq;
+  a.Nc = pl.Nc; a.cmp_block = f.cmp_block; a.cmp_stride = f.cmp_stride;
+  a.cmp_offset = (f.cmp_stride == f.cmp_block ? pl.Nc * f.cmp_block : f.Tk) - f.Tq;
+  a.nq = pl.nq; a.top_k = pl.k_sel; a.bm = f.bm; a.bn = f.bn; a.sel_key_limit = pl.nk * f.bn;
+  a.window = f.window; a.causal = f.causal;
+  a.gate_act = f.gate_act; a.q_dtype = f.q_dtype; a.kv_dtype = pl.dequant ? NSA_BF16 : f.q_dtype;
+  a.scale = f.scale; a.q_scale = f.q_scale; a.k_scale = f.k_scale; a.v_scale = f.v_scale;
+  a.engine = f.engine; a.io_layout = f.io_layout;
+  return a;
 }
 
 }  // namespace nsa
@@ -108,18 +130,62 @@ int nsa_forward(const nsa_forward_args* fa, nsa_stream_t stream) {
     K = ws + pl.o_k16;
     V = ws + pl.o_v16;
   }
-  nsa_fwd_args a = {};
-  a.Q = f.Q; a.K = K; a.V = V; a.Kc = ws + pl.o_kc; a.Vc = ws + pl.o_vc; a.idx = idx; a.gates = f.gates; a.out = f.out;
-  a.B = f.B; a.H = f.H; a.Hkv = f.Hkv; a.Hi = pl.Hi; a.Tq = f.Tq; a.Tk = f.Tk; a.D = f.D; a.offset = f.Tk - f.Tq;
-  a.Nc = pl.Nc; a.cmp_block = f.cmp_block; a.cmp_stride = f.cmp_stride;
-  a.cmp_offset = (f.cmp_stride == f.cmp_block ? pl.Nc * f.cmp_block : f.Tk) - f.Tq;
-  a.nq = pl.nq; a.top_k = pl.k_sel; a.bm = f.bm; a.bn = f.bn; a.sel_key_limit = pl.nk * f.bn;
-  a.window = f.window; a.causal = f.causal;
+  nsa_fwd_args a = attention_args(f, pl, K, V, ws + pl.o_kc, ws + pl.o_vc, idx);
+  a.out = f.out; a.gates = f.gates; a.gate_dtype = f.gate_dtype;
   a.branches = NSA_BRANCH_COMPRESSED | NSA_BRANCH_SELECTED | NSA_BRANCH_SLIDING;
-  a.fused = 1; a.gate_act = f.gate_act; a.q_dtype = f.q_dtype; a.kv_dtype = pl.dequant ? NSA_BF16 : f.q_dtype; a.gate_dtype = f.gate_dtype;
-  a.scale = f.scale; a.q_scale = f.q_scale; a.k_scale = f.k_scale; a.v_scale = f.v_scale;
-  a.engine = f.engine; a.io_layout = f.io_layout;
+  a.fused = 1;
   return nsa_attention_fwd(&a, stream);
+}
+
+int64_t nsa_backward_ws_bytes(const nsa_forward_args* f) {
+  NSA_REQUIRE(f, NSA_ERR_ARG, "backward: NULL argument block");
+  return backward_ws_bytes(*f);
+}
+
+int nsa_forward_train(const nsa_forward_args* fa, void* branch_out, float* branch_lse, int32_t* idx, void* Kc, void* Vc, nsa_stream_t stream) {
+  NSA_REQUIRE(fa, NSA_ERR_ARG, "forward (training): NULL argument block");
+  const nsa_forward_args& f = *fa;
+  ForwardPlan pl;
+  int rc = forward_plan(f, pl);
+  if (rc != NSA_OK) return rc;
+  NSA_REQUIRE(f.Q && f.K && f.V && f.out && branch_out && branch_lse && Kc && Vc && (pl.select ? idx != nullptr : f.idx != nullptr), NSA_ERR_ARG,
+              "forward (training): NULL pointer");
+  NSA_REQUIRE(!fp8(f.q_dtype) && f.io_layout == 0, NSA_ERR_UNSUPPORTED, "forward (training): 16-bit storage in the default layout only");
+  NSA_REQUIRE(!pl.select || (f.ws && f.ws_bytes >= (int64_t)pl.total), NSA_ERR_ARG, "forward (training): needs %lld bytes of workspace, %lld given",
+              (long long)pl.total, (long long)f.ws_bytes);
+  cudaStream_t st = (cudaStream_t)stream;
+  unsigned char* ws = reinterpret_cast<unsigned char*>(f.ws);
+  const int BH = f.B * f.H, BKV = f.B * f.Hkv;
+  PoolJob jobs[4];
+  int n = 0;
+  if (pl.select) {
+    jobs[n++] = {f.Q, ws + pl.o_qb, f.Tq, f.bm, f.bm, pl.nq, BH, 1.f, 0u};
+    jobs[n++] = {f.K, ws + pl.o_kb, f.Tk, f.bn, f.bn, pl.nk, BKV, 1.f, 0u};
+  }
+  jobs[n++] = {f.K, Kc, f.Tk, f.cmp_block, f.cmp_stride, pl.Nc, BKV, 1.f, 0u};
+  jobs[n++] = {f.V, Vc, f.Tk, f.cmp_block, f.cmp_stride, pl.Nc, BKV, 1.f, 0u};
+  if ((rc = pool_mean_multi(jobs, n, f.D, f.q_dtype, st)) != NSA_OK) return rc;
+  if (pl.select && (rc = select_blocks(ws + pl.o_qb, ws + pl.o_kb, idx, f.B, f.H, f.Hkv, pl.nq, pl.nk, f.D, f.top_k, f.bm, f.bn,
+                                       pl.nk * f.bn - pl.nq * f.bm, f.causal, f.scale, f.force_first, f.force_local, f.per_group, f.q_dtype,
+                                       nullptr, st)) != NSA_OK)
+    return rc;
+  const size_t rows = (size_t)BH * f.Tq, bytes = rows * f.D * 2;
+  unsigned char* bo = reinterpret_cast<unsigned char*>(branch_out);
+  for (int br = 0; br < 3; ++br) {
+    nsa_fwd_args a = attention_args(f, pl, f.K, f.V, Kc, Vc, pl.select ? idx : f.idx);
+    a.out = bo + br * bytes; a.lse = branch_lse + br * rows;
+    a.branches = 1 << br;
+    if ((rc = nsa_attention_fwd(&a, stream)) != NSA_OK) return rc;
+  }
+  return combine(bo, bo + bytes, bo + 2 * bytes, f.gates, f.out, (long long)rows, f.D, f.gate_act, f.q_dtype, f.gates ? f.gate_dtype : f.q_dtype,
+                 f.q_dtype, st);
+}
+
+int nsa_backward(const nsa_forward_args* f, const void* dO, const void* branch_out, const float* branch_lse, const int32_t* idx, const void* Kc,
+                 const void* Vc, void* dQ, void* dK, void* dV, void* dgates, nsa_stream_t stream) {
+  NSA_REQUIRE(f, NSA_ERR_ARG, "backward: NULL argument block");
+  NSA_REQUIRE(f->Q && f->K && f->V && dO && branch_out && branch_lse && idx && Kc && Vc && dQ && dK && dV, NSA_ERR_ARG, "backward: NULL pointer");
+  return backward_stream(*f, dO, branch_out, branch_lse, idx, Kc, Vc, dQ, dK, dV, dgates, (cudaStream_t)stream);
 }
 
 }  // extern "C"

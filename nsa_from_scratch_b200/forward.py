@@ -138,6 +138,26 @@ class _CombineFn(torch.autograd.Function):
         return tuple(gr.to(t.dtype) for gr, t in zip(grads, (oc, os_, ow, gl))) + (None,)
 
 
+class _NSAFn(torch.autograd.Function):
+    """The whole forward and its backward, one library call each: the branch outputs and log-sum-exps, the block lists
+    and the pooled keys and values are kept between them."""
+
+    @staticmethod
+    def forward(ctx, Q, K, V, gates, idx, plan):
+        out, branch, lse, idx, pooled = ops.forward_train(Q, K, V, gates, idx, plan)
+        ctx.save_for_backward(Q, K, V, gates, branch, lse, idx, pooled)
+        ctx.plan = plan
+        return out
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, grad_out):
+        Q, K, V, gates, branch, lse, idx, pooled = ctx.saved_tensors
+        dO = ops._dense(grad_out.to(Q.dtype), "dO")
+        dQ, dK, dV, dg = ops.backward(dO, Q, K, V, gates, branch, lse, idx, pooled, ctx.plan)
+        return dQ, dK, dV, dg, None, None
+
+
 def _cfg(cfg, name, default):
     v = getattr(cfg, name, default)
     return default if v is None else v
@@ -181,6 +201,17 @@ def nsa_forward(Q: Tensor, K: Tensor, V: Tensor, cfg, *, gate_logits: Optional[T
     if needs_grad and learned:
         raise NotImplementedError("nsa_forward: pool='learned' is forward-only here (no gradient kernels for the pooling weights)")
     if needs_grad:
+        geometry = _geometry(cfg, float(scale), stride_c)
+        ops._check_forward(Q, K, V, gate_logits, False)
+        if ops.bwd_engine() != L.ENGINE_GENERIC:
+            idx = None if block_indices is None else block_indices.to(torch.int32).contiguous()
+            plan = ops.forward_plan(Q.shape, K.shape, Q.dtype, idx_shape=None if idx is None else idx.shape,
+                                    gate_dtype=None if gate_logits is None else gate_logits.dtype, q_scale=1.0, k_scale=1.0, v_scale=1.0,
+                                    engine=ops.engine(), token_major=False, **geometry)
+            if plan[2] > 0:
+                return _NSAFn.apply(ops._dense(Q, "Q"), ops._dense(K, "K"), ops._dense(V, "V"),
+                                    None if gate_logits is None else ops._dense(gate_logits, "gates"), idx, plan)
+        # shapes that the streaming backward does not take (D = 32, blocks other than 64): branch by branch
         if block_indices is None:
             block_indices = _resolve_from_cfg(Q, K, cfg, float(scale))
         out_c = _CompressedFn.apply(Q, K, V, cfg.block_size_c, cfg.pool, cfg.causal, cfg.scale, stride_c)
@@ -204,17 +235,22 @@ def _gate_act(cfg) -> int:
     raise ValueError(f"unknown gate_activation: {cfg.gate_activation}")
 
 
+def _geometry(cfg, scale, stride_c) -> dict:
+    bc = cfg.block_size_c
+    return dict(causal=bool(cfg.causal), scale=scale, cmp_block=bc, cmp_stride=bc if stride_c is None else int(stride_c),
+                bm=cfg.block_size_m, bn=cfg.block_size_n, window=cfg.window_size, top_k=cfg.top_k,
+                force_first=_cfg(cfg, "force_first", 0), force_local=_cfg(cfg, "force_local", 0),
+                per_group=bool(_cfg(cfg, "select_per_group", False)), gate_act=_gate_act(cfg))
+
+
 def _fused_forward(Q, K, V, cfg, scale, stride_c, gate_logits, block_indices, sq, sk, sv, engine=None,
                    token_major=False, pool_proj=None):
     """block_indices None: chosen inside the call by block means."""
     bc = cfg.block_size_c
     stride = bc if stride_c is None else int(stride_c)
     if pool_proj is None:
-        return ops.forward(
-            Q, K, V, causal=bool(cfg.causal), scale=scale, cmp_block=bc, cmp_stride=stride, bm=cfg.block_size_m, bn=cfg.block_size_n,
-            window=cfg.window_size, top_k=cfg.top_k, force_first=_cfg(cfg, "force_first", 0), force_local=_cfg(cfg, "force_local", 0),
-            per_group=bool(_cfg(cfg, "select_per_group", False)), idx=block_indices, gates=gate_logits, gate_act=_gate_act(cfg),
-            q_scale=sq, k_scale=sk, v_scale=sv, engine=engine, token_major=token_major)
+        return ops.forward(Q, K, V, idx=block_indices, gates=gate_logits, q_scale=sq, k_scale=sk, v_scale=sv, engine=engine,
+                           token_major=token_major, **_geometry(cfg, scale, stride_c))
     if block_indices is None:
         block_indices = _resolve_from_cfg(Q, K, cfg, scale, sq, sk)
     Kc = ops.pool_learned(K, pool_proj[0], bc, stride)

@@ -38,6 +38,10 @@ def set_bwd_engine(name: str) -> None:
     _BWD_ENGINE = {"auto": L.ENGINE_AUTO, "generic": L.ENGINE_GENERIC, "tcgen05": L.ENGINE_TCGEN05}[name]
 
 
+def bwd_engine() -> int:
+    return _BWD_ENGINE
+
+
 def device_status() -> None:
     """Synchronise the current stream and raise if a kernel gave up on a bounded device-side wait."""
     L.check(L.load().nsa_device_status(L.stream_ptr()), "nsa_device_status")
@@ -274,62 +278,81 @@ def attention_fwd(
     return out, lse
 
 
-# nsa_forward_args of the problems seen so far, pointers left out: (bytes of the struct, workspace bytes)
+# nsa_forward_args of the problems seen so far, pointers left out: (bytes of the struct, workspace bytes of the forward,
+# of the backward (0: not taken), shape of the block lists, pooled tokens)
 _forward_plans: dict = {}
 
 
-def forward(Q: Tensor, K: Tensor, V: Tensor, *, causal: bool, scale: float, cmp_block: int, cmp_stride: int, bm: int, bn: int, window: int,
-            top_k: int, force_first: int = 0, force_local: int = 0, per_group: bool = False, idx: Optional[Tensor] = None,
-            gates: Optional[Tensor] = None, gate_act: int = L.GATE_SIGMOID, q_scale: float = 1.0, k_scale: float = 1.0,
-            v_scale: float = 1.0, engine: Optional[int] = None, token_major: bool = False) -> Tensor:
-    """The whole forward (window means, selection unless `idx` is given, the fused launch) as one library call."""
-    _need_cuda(Q, K, V)
-    q_shape, k_shape, dtype = Q.shape, K.shape, Q.dtype
+def forward_plan(q_shape, k_shape, dtype, *, causal: bool, scale: float, cmp_block: int, cmp_stride: int, bm: int, bn: int, window: int,
+                 top_k: int, force_first: int, force_local: int, per_group: bool, idx_shape, gate_dtype, gate_act: int, q_scale: float,
+                 k_scale: float, v_scale: float, engine: int, token_major: bool):
+    key = (q_shape, k_shape, dtype, causal, scale, cmp_block, cmp_stride, bm, bn, window, top_k, force_first, force_local, per_group,
+           idx_shape, gate_dtype, gate_act, q_scale, k_scale, v_scale, engine, token_major)
+    plan = _forward_plans.get(key)
+    if plan is not None:
+        return plan
     B, H, Tq, D = q_shape
+    Hkv, Tk = k_shape[1], k_shape[2]
+    if k_shape != (B, Hkv, Tk, D):
+        raise ValueError(f"K/V shapes {tuple(k_shape)} do not match Q {tuple(q_shape)}")
+    if H % Hkv:
+        raise ValueError(f"query heads {H} not a multiple of KV heads {Hkv}")
+    a = L.ForwardArgs()
+    a.B, a.H, a.Hkv, a.Tq, a.Tk, a.D = B, H, Hkv, Tq, Tk, D
+    a.top_k, a.force_first, a.force_local, a.per_group = int(top_k), int(force_first), int(force_local), int(per_group)
+    nq, nk = (Tq + bm - 1) // bm, (Tk + bn - 1) // bn
+    if idx_shape is not None:
+        if len(idx_shape) != 4 or idx_shape[0] != B or idx_shape[1] not in (H, Hkv) or idx_shape[2] != nq:
+            raise ValueError(f"block_indices shape {tuple(idx_shape)} does not match (B={B}, H={H}|{Hkv}, nq={nq}, k)")
+        a.has_idx, a.Hi, a.top_k = 1, idx_shape[1], idx_shape[3]
+    else:
+        idx_shape = (B, Hkv if per_group else H, nq, min(int(top_k), nk))
+    a.cmp_block, a.cmp_stride, a.bm, a.bn, a.window, a.causal = cmp_block, cmp_stride, bm, bn, int(window), int(causal)
+    a.gate_act, a.q_dtype, a.engine = gate_act, L.dtype_code(dtype), engine
+    a.gate_dtype = 0 if gate_dtype is None else L.dtype_code(gate_dtype)
+    a.io_layout = (L.IO_OUT_BTHD | L.IO_GATES_BTHD) if token_major else 0
+    a.scale, a.q_scale, a.k_scale, a.v_scale = float(scale), float(q_scale), float(k_scale), float(v_scale)
+    lib = L.load()
+    need = int(lib.nsa_forward_ws_bytes(C.byref(a)))
+    if need < 0:
+        L.check(need, "nsa_forward")
+    if len(_forward_plans) >= 256:           # a program meets few shapes; one that meets many starts over
+        _forward_plans.clear()
+    plan = _forward_plans[key] = (bytes(a), need, int(lib.nsa_backward_ws_bytes(C.byref(a))), idx_shape, n_pooled(Tk, cmp_block, cmp_stride))
+    return plan
+
+
+def _check_forward(Q: Tensor, K: Tensor, V: Tensor, gates: Optional[Tensor], token_major: bool) -> None:
+    _need_cuda(Q, K, V)
+    if V.shape != K.shape:
+        raise ValueError(f"K/V shapes {tuple(K.shape)}/{tuple(V.shape)} do not match Q {tuple(Q.shape)}")
+    if V.dtype != Q.dtype or K.dtype != Q.dtype:
+        raise TypeError("Q, K, V must share a dtype")
+    if gates is not None:
+        B, H, Tq, _ = Q.shape
+        want = (B, Tq, H, 3) if token_major else (B, H, Tq, 3)
+        if gates.shape != want:
+            raise ValueError(f"gate_logits shape {tuple(gates.shape)} != {want}")
+
+
+def forward(Q: Tensor, K: Tensor, V: Tensor, *, idx: Optional[Tensor] = None, gates: Optional[Tensor] = None, q_scale: float = 1.0,
+            k_scale: float = 1.0, v_scale: float = 1.0, engine: Optional[int] = None, token_major: bool = False, **geometry) -> Tensor:
+    """The whole forward (window means, selection unless `idx` is given, the fused launch) as one library call.
+    `geometry`: causal, scale, cmp_block, cmp_stride, bm, bn, window, top_k, force_first, force_local, per_group, gate_act."""
+    _check_forward(Q, K, V, gates, token_major)
     Q, K, V = _dense(Q, "Q"), _dense(K, "K"), _dense(V, "V")
     if idx is not None:
         idx = idx.to(torch.int32).contiguous()
     if gates is not None:
         gates = _dense(gates, "gates")
-    eng = _ENGINE if engine is None else engine
-    key = (q_shape, k_shape, dtype, causal, scale, cmp_block, cmp_stride, bm, bn, window, top_k, force_first, force_local, per_group,
-           None if idx is None else idx.shape, None if gates is None else gates.dtype, gate_act, q_scale, k_scale, v_scale, eng,
-           token_major)
-    plan = _forward_plans.get(key)
-    if V.shape != k_shape or V.dtype != dtype or K.dtype != dtype:
-        if V.shape != k_shape:
-            raise ValueError(f"K/V shapes {tuple(k_shape)}/{tuple(V.shape)} do not match Q {tuple(q_shape)}")
-        raise TypeError("Q, K, V must share a dtype")
-    if gates is not None and gates.shape != ((B, Tq, H, 3) if token_major else (B, H, Tq, 3)):
-        raise ValueError(f"gate_logits shape {tuple(gates.shape)} != {(B, Tq, H, 3) if token_major else (B, H, Tq, 3)}")
-    if plan is None:
-        Hkv, Tk = k_shape[1], k_shape[2]
-        if k_shape != (B, Hkv, Tk, D):
-            raise ValueError(f"K/V shapes {tuple(k_shape)}/{tuple(V.shape)} do not match Q {tuple(q_shape)}")
-        if H % Hkv:
-            raise ValueError(f"query heads {H} not a multiple of KV heads {Hkv}")
-        a = L.ForwardArgs()
-        a.B, a.H, a.Hkv, a.Tq, a.Tk, a.D = B, H, Hkv, Tq, Tk, D
-        a.top_k, a.force_first, a.force_local, a.per_group = int(top_k), int(force_first), int(force_local), int(per_group)
-        if idx is not None:
-            nq = (Tq + bm - 1) // bm
-            if idx.dim() != 4 or idx.shape[0] != B or idx.shape[1] not in (H, Hkv) or idx.shape[2] != nq:
-                raise ValueError(f"block_indices shape {tuple(idx.shape)} does not match (B={B}, H={H}|{Hkv}, nq={nq}, k)")
-            a.has_idx, a.Hi, a.top_k = 1, idx.shape[1], idx.shape[3]
-        a.cmp_block, a.cmp_stride, a.bm, a.bn, a.window, a.causal = cmp_block, cmp_stride, bm, bn, int(window), int(causal)
-        a.gate_act, a.q_dtype, a.engine = gate_act, L.dtype_code(dtype), eng
-        a.gate_dtype = 0 if gates is None else L.dtype_code(gates.dtype)
-        a.io_layout = (L.IO_OUT_BTHD | L.IO_GATES_BTHD) if token_major else 0
-        a.scale, a.q_scale, a.k_scale, a.v_scale = float(scale), float(q_scale), float(k_scale), float(v_scale)
-        need = int(L.load().nsa_forward_ws_bytes(C.byref(a)))
-        if need < 0:
-            L.check(need, "nsa_forward")
-        if len(_forward_plans) >= 256:       # a program meets few shapes; one that meets many starts over
-            _forward_plans.clear()
-        plan = _forward_plans[key] = (bytes(a), need)
+    dtype = Q.dtype
+    plan = forward_plan(Q.shape, K.shape, dtype, idx_shape=None if idx is None else idx.shape, gate_dtype=None if gates is None else gates.dtype,
+                        q_scale=q_scale, k_scale=k_scale, v_scale=v_scale, engine=_ENGINE if engine is None else engine,
+                        token_major=token_major, **geometry)
     a = L.ForwardArgs.from_buffer_copy(plan[0])
+    B, H, Tq, D = Q.shape
     dev = Q.device
-    out = torch.empty((B, Tq, H, D) if token_major else q_shape, device=dev, dtype=torch.bfloat16 if dtype in _8 else dtype)
+    out = torch.empty((B, Tq, H, D) if token_major else (B, H, Tq, D), device=dev, dtype=torch.bfloat16 if dtype in _8 else dtype)
     ws = torch.empty(plan[1], device=dev, dtype=torch.uint8)
     a.Q, a.K, a.V, a.out, a.ws, a.ws_bytes = Q.data_ptr(), K.data_ptr(), V.data_ptr(), out.data_ptr(), ws.data_ptr(), plan[1]
     if gates is not None:
@@ -339,6 +362,47 @@ def forward(Q: Tensor, K: Tensor, V: Tensor, *, causal: bool, scale: float, cmp_
     with L.on_device(Q):
         L.check(L.load().nsa_forward(C.byref(a), L.stream_ptr()), "nsa_forward")
     return out
+
+
+def forward_train(Q: Tensor, K: Tensor, V: Tensor, gates: Optional[Tensor], idx: Optional[Tensor], plan):
+    """The forward that keeps what `backward` needs; dense operands, `plan` from forward_plan.
+    Returns (out, branch outputs [3,B,H,Tq,D], their log-sum-exps [3,B,H,Tq], block lists, pooled K and V [2,B,Hkv,Nc,D])."""
+    a = L.ForwardArgs.from_buffer_copy(plan[0])
+    B, H, Tq, D = Q.shape
+    dev = Q.device
+    out = torch.empty((B, H, Tq, D), device=dev, dtype=Q.dtype)
+    branch = torch.empty((3, B, H, Tq, D), device=dev, dtype=Q.dtype)
+    lse = torch.empty((3, B, H, Tq), device=dev, dtype=torch.float32)
+    pooled = torch.empty((2, B, K.shape[1], plan[4], D), device=dev, dtype=Q.dtype)
+    ws = torch.empty(plan[1], device=dev, dtype=torch.uint8)
+    if idx is None:
+        idx = torch.empty(plan[3], device=dev, dtype=torch.int32)
+    else:
+        a.idx = idx.data_ptr()
+    a.Q, a.K, a.V, a.out, a.ws, a.ws_bytes = Q.data_ptr(), K.data_ptr(), V.data_ptr(), out.data_ptr(), ws.data_ptr(), plan[1]
+    a.gates = L.ptr(gates)
+    pk = pooled.data_ptr()
+    with L.on_device(Q):
+        L.check(L.load().nsa_forward_train(C.byref(a), branch.data_ptr(), lse.data_ptr(), idx.data_ptr(), pk, pk + pooled.numel() // 2 * 2,
+                                           L.stream_ptr()), "nsa_forward_train")
+    return out, branch, lse, idx, pooled
+
+
+def backward(dO: Tensor, Q: Tensor, K: Tensor, V: Tensor, gates: Optional[Tensor], branch: Tensor, lse: Tensor, idx: Tensor, pooled: Tensor, plan):
+    """(dQ, dK, dV, dgates or None) of `forward_train`, one library call."""
+    a = L.ForwardArgs.from_buffer_copy(plan[0])
+    dev = Q.device
+    dQ, dK, dV = torch.empty_like(Q), torch.empty_like(K), torch.empty_like(V)
+    dg = None if gates is None else torch.empty_like(gates)
+    ws = torch.empty(plan[2], device=dev, dtype=torch.uint8)
+    a.Q, a.K, a.V, a.ws, a.ws_bytes = Q.data_ptr(), K.data_ptr(), V.data_ptr(), ws.data_ptr(), plan[2]
+    a.gates = L.ptr(gates)
+    pk = pooled.data_ptr()
+    with L.on_device(Q):
+        L.check(L.load().nsa_backward(C.byref(a), dO.data_ptr(), branch.data_ptr(), lse.data_ptr(), idx.data_ptr(), pk,
+                                      pk + pooled.numel() // 2 * 2, dQ.data_ptr(), dK.data_ptr(), dV.data_ptr(), L.ptr(dg), L.stream_ptr()),
+                "nsa_backward")
+    return dQ, dK, dV, dg
 
 
 def bwd_delta(dO: Tensor, O: Tensor) -> Tensor:

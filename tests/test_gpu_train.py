@@ -1,0 +1,62 @@
+"""The whole forward's backward (streaming kernels over all branches) against autograd through the fp32 oracle.
+Tolerance: max-abs <= 2e-2 * max(1, max|reference|), as for the other 16-bit gradients: an entry is a sum over
+hundreds of rows whose operands and result are rounded to 8 (bf16) or 11 bits."""
+import pytest
+import torch
+
+from helpers import make_qkv, max_abs
+from oracle import nsa_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def nsa():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import nsa_from_scratch_b200 as pkg
+    return pkg
+
+
+# B, H, Hkv, Tq, Tk, D, top_k, window, (cmp block, stride), one list per KV head, dtype, causal, gates, gate dtype
+CASES = [
+    (1, 2, 2, 256, 256, 64, 3, 64, (64, 64), False, torch.bfloat16, True, "sigmoid", torch.bfloat16),   # a KV head per head
+    (2, 3, 1, 200, 200, 64, 3, 100, (32, 16), True, torch.bfloat16, True, "softmax", torch.float32),    # odd heads, ragged
+    (1, 4, 2, 130, 333, 128, 4, 65, (32, 16), True, torch.float16, True, "sigmoid", torch.float32),     # Tq < Tk
+    (1, 4, 1, 192, 192, 128, 5, 70, (32, 16), False, torch.bfloat16, True, "sigmoid", torch.bfloat16),  # lists per head
+    (1, 2, 1, 192, 256, 64, 2, 50, (32, 16), True, torch.bfloat16, False, "sigmoid", torch.bfloat16),   # not causal
+    (1, 1, 1, 65, 65, 64, 16, 512, (64, 64), False, torch.float16, True, "softmax", torch.float16),     # one row in the last block
+    (1, 16, 1, 640, 640, 64, 4, 128, (32, 16), True, torch.bfloat16, True, "sigmoid", None),            # several segments, no gates
+]
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_gradients_vs_oracle(nsa, case):
+    from nsa_from_scratch_b200 import ops
+    B, H, Hkv, Tq, Tk, D, k, W, (bc, st), group, dt, causal, act, gdt = case
+    Q, K, V, g = make_qkv(31, B, H, Hkv, Tq, Tk, D, dtype=dt)
+    gates = torch.randn(B, H, Tq, 3, generator=g).to(gdt) if gdt is not None else None
+    dO = torch.randn(B, H, Tq, D, generator=g).to(dt)
+    ff, fl = (1, 1) if group else (0, 0)
+    cfg = nsa.NSAConfig(block_size_c=bc, stride_c=None if st == bc else st, top_k=k, window_size=W, causal=causal, gate_activation=act,
+                        select_per_group=group, force_first=ff, force_local=fl)
+    idx = O.select_blocks(Q, K, top_k=k, causal=causal, force_first=ff, force_local=fl, group_shared=group)
+    leaves = [t.float().clone().requires_grad_(True) for t in (Q, K, V)]
+    logits = (torch.zeros(B, H, Tq, 3) if gates is None else gates.float()).clone().requires_grad_(True)
+    oc = O.compressed_attention(*leaves, block_size_c=bc, stride_c=None if st == bc else st, causal=causal)[0]
+    os_ = O.selected_attention(*leaves, block_indices=idx, causal=causal)[0]
+    ow = O.sliding_attention(*leaves, window_size=W, causal=causal)[0]
+    gv = torch.sigmoid(logits) if act == "sigmoid" else torch.softmax(logits, -1)
+    ref_out = gv[..., 0:1] * oc + gv[..., 1:2] * os_ + gv[..., 2:3] * ow
+    ref = torch.autograd.grad(ref_out, [*leaves, logits], dO.float())
+    dev = [t.cuda().requires_grad_(True) for t in (Q, K, V)] + ([] if gates is None else [gates.cuda().requires_grad_(True)])
+    out = nsa.nsa_forward(*dev[:3], cfg, gate_logits=None if gates is None else dev[3])
+    assert out.dtype == dt and max_abs(out.detach(), ref_out.detach()) <= 2e-2
+    got = torch.autograd.grad(out, dev, dO.cuda())
+    ops.device_status()
+    for name, a, r in zip(("dQ", "dK", "dV", "dgates"), got, ref):
+        assert a.shape == r.shape
+        err, mag = max_abs(a, r), float(r.abs().max())
+        assert err <= 2e-2 * max(1.0, mag), (name, err, mag)
+    again = torch.autograd.grad(nsa.nsa_forward(*dev[:3], cfg, gate_logits=None if gates is None else dev[3]), dev, dO.cuda())
+    assert torch.equal(again[0], got[0])                 # dQ is formed in a fixed order
