@@ -236,6 +236,27 @@ int64_t nsa_backward_ws_bytes(const nsa_forward_args* args);
 int nsa_backward(const nsa_forward_args* args, const void* dO, const void* branch_out, const float* branch_lse, const int32_t* idx,
                  const void* Kc, const void* Vc, void* dQ, void* dK, void* dV, void* dgates, nsa_stream_t stream);
 
+/* One decoding step against a KV cache (nsa_cache_append keeps it): q [B,H,Tq,D] are the queries of the last Tq of
+ * `len` filled positions; K/V [B,Hkv,max_len,D], pooled Kc/Vc [B,Hkv,nc_alloc,D], block means Kb [B,Hkv,nk_alloc,D].
+ * Scores, selection, the three branches and the gated combine: what nsa_forward returns for these queries over the
+ * filled prefix.  dyn_len != NULL: the length is read on the device (len is then ignored; the grid is sized for
+ * max_len), so that a captured step stays valid as the cache grows.  ws: nsa_decode_ws_bytes(&args) bytes,
+ * 256-byte aligned; 0 means that the shape is not taken (D in {64,128}, 16-bit storage, bm = bn = 64, top_k <= 64,
+ * at most 64 query rows per KV head): nsa_select_blocks + nsa_attention_fwd serve those. */
+typedef struct nsa_decode_args {
+  const void *Q, *K, *V, *Kc, *Vc, *Kb, *gates;
+  void *out, *ws;
+  const int32_t* dyn_len;
+  int64_t ws_bytes;
+  int32_t B, H, Hkv, Tq, len, D, max_len, nc_alloc, nk_alloc;
+  int32_t cmp_block, cmp_stride, bm, bn, top_k, window, force_first, force_local, per_group;
+  int32_t gate_act, dtype, gate_dtype;
+  float scale;
+} nsa_decode_args;
+
+int64_t nsa_decode_ws_bytes(const nsa_decode_args* args);
+int nsa_decode(const nsa_decode_args* args, nsa_stream_t stream);
+
 /* Synchronises `stream`, then reports whether any kernel launched so far gave up on one of
  * its bounded device-side waits: NSA_OK, or NSA_ERR_DEVICE (and the condition is cleared).
  * No counterpart in the reference (its kernels have no device-side waits). */

@@ -87,6 +87,19 @@ class ForwardArgs(C.Structure):
     ]
 
 
+class DecodeArgs(C.Structure):
+    """Mirror of `struct nsa_decode_args`."""
+    _fields_ = [
+        ("Q", C.c_void_p), ("K", C.c_void_p), ("V", C.c_void_p), ("Kc", C.c_void_p), ("Vc", C.c_void_p), ("Kb", C.c_void_p),
+        ("gates", C.c_void_p), ("out", C.c_void_p), ("ws", C.c_void_p), ("dyn_len", C.c_void_p), ("ws_bytes", C.c_int64),
+        ("B", C.c_int32), ("H", C.c_int32), ("Hkv", C.c_int32), ("Tq", C.c_int32), ("len", C.c_int32), ("D", C.c_int32),
+        ("max_len", C.c_int32), ("nc_alloc", C.c_int32), ("nk_alloc", C.c_int32),
+        ("cmp_block", C.c_int32), ("cmp_stride", C.c_int32), ("bm", C.c_int32), ("bn", C.c_int32), ("top_k", C.c_int32),
+        ("window", C.c_int32), ("force_first", C.c_int32), ("force_local", C.c_int32), ("per_group", C.c_int32),
+        ("gate_act", C.c_int32), ("dtype", C.c_int32), ("gate_dtype", C.c_int32), ("scale", C.c_float),
+    ]
+
+
 _vp, _i, _f, _i64 = C.c_void_p, C.c_int, C.c_float, C.c_int64
 
 PROTOTYPES = {
@@ -105,6 +118,8 @@ PROTOTYPES = {
     "nsa_forward_train": (_i, [C.POINTER(ForwardArgs)] + [_vp] * 6),
     "nsa_backward_ws_bytes": (_i64, [C.POINTER(ForwardArgs)]),
     "nsa_backward": (_i, [C.POINTER(ForwardArgs)] + [_vp] * 11),
+    "nsa_decode_ws_bytes": (_i64, [C.POINTER(DecodeArgs)]),
+    "nsa_decode": (_i, [C.POINTER(DecodeArgs), _vp]),
     "nsa_device_status": (_i, [_vp]),
     "nsa_debug_set_device_status": (_i, [_i, _i]),
     "nsa_compressed_attention_static": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp]),

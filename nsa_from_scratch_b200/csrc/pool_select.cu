@@ -172,14 +172,15 @@ int pool_mean(const void* x, void* out, int B, int H, int T, int D, int block, i
 // windows and selection-block means that contain a new row are recomputed with pool_mean_kernel's arithmetic
 // (fp32 sum in row order, divide by the window size, one rounding).  Rows at or past `filled` are read from
 // the new tensors, so nothing in the launch depends on another thread's copy.
-// One thread = 8 columns of one item; items of a slab: t_new row copies, nw pooled windows, nbk block means.
+// One thread = 8 columns of one item; items of a slab: t_new row copies, nw pooled windows of K and of V, nbk block means.
 template <typename T>
-__global__ void __launch_bounds__(256) cache_append_kernel(const T* __restrict__ k_new, const T* __restrict__ v_new,
+__global__ void __launch_bounds__(64) cache_append_kernel(const T* __restrict__ k_new, const T* __restrict__ v_new,
                                                            T* __restrict__ K, T* __restrict__ V, T* __restrict__ Kc,
                                                            T* __restrict__ Vc, T* __restrict__ Kb, int D, int t_new,
                                                            int filled, int max_len, int nc_alloc, int nb_alloc, int cblock,
                                                            int cstride, int c0, int nw, int sblock, int b0, int nbk,
                                                            const int32_t* __restrict__ dyn_filled) {
+  grid_dep_wait();
   const int CH = D / 8;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (dyn_filled != nullptr) {
@@ -194,52 +195,53 @@ __global__ void __launch_bounds__(256) cache_append_kernel(const T* __restrict__
     b0 = filled / sblock;
     nbk = min((T1d + sblock - 1) / sblock, nb_alloc) - b0;
   }
-  const long long items = (long long)t_new + nw + nbk;
+  const long long items = (long long)t_new + 2LL * nw + nbk;
   if (i >= items * CH) return;
   const int item = (int)(i / CH), ch = (int)(i % CH);
   const size_t slab = blockIdx.y;
   const int T1 = filled + t_new;
-  auto row8 = [&](const T* cache, const T* fresh, int r) {
-    const T* p = r >= filled ? fresh + (slab * t_new + (r - filled)) * D : cache + (slab * max_len + r) * D;
-    return *reinterpret_cast<const uint4*>(p + ch * 8);
-  };
-  auto mean8 = [&](const T* cache, const T* fresh, int r0, int block) {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const int r1 = min(r0 + block, T1);
-    for (int rb = r0; rb < r1; rb += 8) {                  // eight rows' loads in flight, added in row order
-      uint4 raw[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) raw[j] = rb + j < r1 ? row8(cache, fresh, rb + j) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (rb + j < r1) {
-          const uint32_t w[4] = {raw[j].x, raw[j].y, raw[j].z, raw[j].w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 f = Elem<T>::unpack(w[e]);
-            acc[2 * e] += f.x;
-            acc[2 * e + 1] += f.y;
-          }
-        }
-      }
-    }
-    const float n = (float)block;
-    return make_uint4(Elem<T>::pack(__fdiv_rn(acc[0], n), __fdiv_rn(acc[1], n)), Elem<T>::pack(__fdiv_rn(acc[2], n), __fdiv_rn(acc[3], n)),
-                      Elem<T>::pack(__fdiv_rn(acc[4], n), __fdiv_rn(acc[5], n)), Elem<T>::pack(__fdiv_rn(acc[6], n), __fdiv_rn(acc[7], n)));
-  };
   if (item < t_new) {
     const size_t dst = (slab * max_len + filled + item) * D + ch * 8, src = (slab * t_new + item) * D + ch * 8;
     *reinterpret_cast<uint4*>(K + dst) = *reinterpret_cast<const uint4*>(k_new + src);
     *reinterpret_cast<uint4*>(V + dst) = *reinterpret_cast<const uint4*>(v_new + src);
-  } else if (item < t_new + nw) {
-    const int c = c0 + (item - t_new);
-    const size_t dst = (slab * nc_alloc + c) * D + ch * 8;
-    *reinterpret_cast<uint4*>(Kc + dst) = mean8(K, k_new, c * cstride, cblock);
-    *reinterpret_cast<uint4*>(Vc + dst) = mean8(V, v_new, c * cstride, cblock);
-  } else {
-    const int bb = b0 + (item - t_new - nw);
-    *reinterpret_cast<uint4*>(Kb + (slab * nb_alloc + bb) * D + ch * 8) = mean8(K, k_new, bb * sblock, sblock);
+    return;
   }
+  // one window or block mean: rows r0 .. r1-1, 32 of them fetched (from a clamped address, so that no load waits for a
+  // branch) before any is added
+  const bool win = item < t_new + 2 * nw;
+  const int w = win ? (item - t_new) >> 1 : item - t_new - 2 * nw;
+  const bool isv = win && ((item - t_new) & 1);
+  const T* cache = (isv ? V : K) + slab * max_len * D + ch * 8;
+  const T* fresh = (isv ? v_new : k_new) + slab * t_new * D + ch * 8;
+  const int block = win ? cblock : sblock;
+  const int r0 = win ? (c0 + w) * cstride : (b0 + w) * sblock, r1 = min(r0 + block, T1);
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int rb = r0; rb < r1; rb += 32) {
+    uint4 raw[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const int r = min(rb + j, r1 - 1);
+      const T* q = r >= filled ? fresh + (size_t)(r - filled) * D : cache + (size_t)r * D;
+      raw[j] = __ldcg(reinterpret_cast<const uint4*>(q));
+    }
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      if (rb + j < r1) {
+        const uint32_t u[4] = {raw[j].x, raw[j].y, raw[j].z, raw[j].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = Elem<T>::unpack(u[e]);
+          acc[2 * e] += f.x;
+          acc[2 * e + 1] += f.y;
+        }
+      }
+    }
+  }
+  const float n = (float)block;
+  const uint4 m = make_uint4(Elem<T>::pack(__fdiv_rn(acc[0], n), __fdiv_rn(acc[1], n)), Elem<T>::pack(__fdiv_rn(acc[2], n), __fdiv_rn(acc[3], n)),
+                             Elem<T>::pack(__fdiv_rn(acc[4], n), __fdiv_rn(acc[5], n)), Elem<T>::pack(__fdiv_rn(acc[6], n), __fdiv_rn(acc[7], n)));
+  T* dst = win ? (isv ? Vc : Kc) + (slab * nc_alloc + c0 + w) * D : Kb + (slab * nb_alloc + b0 + w) * D;
+  *reinterpret_cast<uint4*>(dst + ch * 8) = m;
 }
 
 __global__ void cache_advance_kernel(int32_t* filled, int t_new, int max_len) {
@@ -271,15 +273,17 @@ int cache_append(const void* k_new, const void* v_new, void* K, void* V, void* K
     NSA_REQUIRE(c0 + nw <= nc_alloc && b0 + nbk <= nb_alloc, NSA_ERR_ARG, "cache append: pooled (%d) or block-mean (%d) allocation too small",
                 nc_alloc, nb_alloc);
   }
-  const long long threads = ((long long)t_new + nw + nbk) * (D / 8);
-  dim3 grid((unsigned)((threads + 255) / 256), (unsigned)(B * Hkv));
+  const long long threads = ((long long)t_new + 2LL * nw + nbk) * (D / 8);
+  dim3 grid((unsigned)((threads + 63) / 64), (unsigned)(B * Hkv));
+  int rc;
 #define NSA_APPEND(TT)                                                                                                  \
-  cache_append_kernel<TT><<<grid, 256, 0, st>>>((const TT*)k_new, (const TT*)v_new, (TT*)K, (TT*)V, (TT*)Kc, (TT*)Vc, (TT*)Kb, D, \
-                                                t_new, filled, max_len, nc_alloc, nb_alloc, cblock, cstride, c0, nw, sblock, b0, nbk, filled_dev)
+  rc = launch_pdl("cache_append", cache_append_kernel<TT>, grid, 64, 0, st, (const TT*)k_new, (const TT*)v_new, (TT*)K, (TT*)V, (TT*)Kc, \
+                  (TT*)Vc, (TT*)Kb, D, t_new, filled, max_len, nc_alloc, nb_alloc, cblock, cstride, c0, nw, sblock, b0, nbk, filled_dev)
   if (dtype == NSA_BF16) NSA_APPEND(__nv_bfloat16);
   else if (dtype == NSA_FP16) NSA_APPEND(__half);
   else return fail(NSA_ERR_UNSUPPORTED, "cache append: dtype %d", dtype);
 #undef NSA_APPEND
+  if (rc != NSA_OK) return rc;
   if (filled_dev != nullptr) cache_advance_kernel<<<1, 32, 0, st>>>(filled_dev, t_new, max_len);
   return launch_status("cache_append");
 }

@@ -11,6 +11,7 @@ cache starts zero-filled so that they are finite.)
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import Optional
 
 import torch
@@ -43,6 +44,9 @@ class KVCache:
         self.length = 0
         self.filled_dev: Optional[Tensor] = None    # device copy of `length`, kept once a GraphedDecoder asks for it
 
+    def _ptrs(self):
+        return self.K.data_ptr(), self.V.data_ptr(), self.Kc.data_ptr(), self.Vc.data_ptr(), self.Kb.data_ptr()
+
     def n_pooled(self, T: int) -> int:
         if self.stride == self.bc:
             return _cdiv(T, self.bc)
@@ -67,12 +71,44 @@ class KVCache:
         if k.shape != (B, Hkv, t, D) or v.shape != k.shape or k.dtype != self.K.dtype or v.dtype != self.K.dtype:
             raise ValueError(f"KVCache.append: expected [{B},{Hkv},t,{D}] {self.K.dtype} tensors, got {tuple(k.shape)} {k.dtype}")
         # one launch: rows into K/V, and every pooled window / selection-block mean that contains a new row
-        with torch.cuda.device(self.K.device):
-            L.check(L.load().nsa_cache_append(k.data_ptr(), v.data_ptr(), self.K.data_ptr(), self.V.data_ptr(), self.Kc.data_ptr(),
-                                              self.Vc.data_ptr(), self.Kb.data_ptr(), B, Hkv, D, t, T0, self.max_len,
+        with L.on_device(self.K):
+            L.check(L.load().nsa_cache_append(k.data_ptr(), v.data_ptr(), *self._ptrs(), B, Hkv, D, t, T0, self.max_len,
                                               self.Kc.shape[2], self.Kb.shape[2], self.bc, self.stride, self.bn,
                                               L.dtype_code(self.K.dtype), L.stream_ptr()), "nsa_cache_append")
         self._set_length(T1)
+
+
+def _step(q: Tensor, cache: KVCache, gates: Optional[Tensor], scale: float, dyn_len: Optional[Tensor] = None) -> Optional[Tensor]:
+    """The step as one library call (nsa_decode); None where that path does not take the shape."""
+    if ops.engine() != L.ENGINE_AUTO or q.dtype != cache.K.dtype:
+        return None
+    cfg = cache.cfg
+    B, H, Tq, D = q.shape
+    _, Hkv, _, Dk = cache.K.shape
+    if D != Dk or H % Hkv or B != cache.K.shape[0]:
+        raise ValueError(f"nsa_decode: q {tuple(q.shape)} does not match the cache {tuple(cache.K.shape)}")
+    if gates is not None and gates.shape != (B, H, Tq, 3):
+        raise ValueError(f"gate_logits shape {tuple(gates.shape)} != {(B, H, Tq, 3)}")
+    ops._need_cuda(q)
+    q = ops._dense(q, "q")
+    gates = None if gates is None else ops._dense(gates, "gates")
+    kp, vp, kcp, vcp, kbp = cache._ptrs()
+    a = L.DecodeArgs(q.data_ptr(), kp, vp, kcp, vcp, kbp, L.ptr(gates), None, None, L.ptr(dyn_len), 0,
+                     B, H, Hkv, Tq, cache.length, D, cache.max_len, cache.Kc.shape[2], cache.Kb.shape[2],
+                     cache.bc, cache.stride, cfg.block_size_m, cache.bn, cfg.top_k, cfg.window_size, _cfg(cfg, "force_first", 0),
+                     _cfg(cfg, "force_local", 0), int(bool(_cfg(cfg, "select_per_group", False))),
+                     L.GATE_SOFTMAX if cfg.gate_activation == "softmax" else L.GATE_SIGMOID, L.dtype_code(q.dtype),
+                     0 if gates is None else L.dtype_code(gates.dtype), scale)
+    lib = L.load()
+    need = lib.nsa_decode_ws_bytes(C.byref(a))
+    if need <= 0:
+        return None
+    out = torch.empty((B, H, Tq, D), device=q.device, dtype=q.dtype)
+    ws = torch.empty(need, device=q.device, dtype=torch.uint8)
+    a.out, a.ws, a.ws_bytes = out.data_ptr(), ws.data_ptr(), need
+    with L.on_device(q):
+        L.check(lib.nsa_decode(C.byref(a), L.stream_ptr()), "nsa_decode")
+    return out
 
 
 def _split_ways(B: int, H: int, Hkv: int, Tq: int, n_pooled: int) -> int:
@@ -96,6 +132,10 @@ def nsa_decode(q: Tensor, cache: KVCache, *, gate_logits: Optional[Tensor] = Non
         raise ValueError(f"nsa_decode: {Tq} queries but only {Tk} cached positions")
     scale = float(cfg.scale if cfg.scale is not None else 1.0 / (D ** 0.5))
     bm, bn = int(cfg.block_size_m), cache.bn
+    if nsplit is None:
+        out = _step(q, cache, gate_logits, scale)
+        if out is not None:
+            return out
     Qb = ops.pool_mean(q, bm, bm)
     idx = ops.select_blocks_from_means(
         Qb, cache.Kb, top_k=cfg.top_k, bm=bm, bn=bn, offset=_cdiv(Tk, bn) * bn - _cdiv(Tq, bm) * bm, causal=True, scale=scale,
@@ -131,6 +171,7 @@ class GraphedDecoder:
             cache.filled_dev = torch.full((1,), cache.length, dtype=torch.int32, device=dev)
         # the grid is part of the graph: split as for a full cache
         self.nsplit = _split_ways(B, n_heads, Hkv, self.t, cache.n_pooled(cache.max_len)) if nsplit is None else int(nsplit)
+        self._ask_split = nsplit
         self.scale = float(cfg.scale if cfg.scale is not None else 1.0 / (D ** 0.5))
         start = cache.length
         if start + self.t > cache.max_len:
@@ -158,6 +199,10 @@ class GraphedDecoder:
                                              c.Vc.data_ptr(), c.Kb.data_ptr(), B, Hkv, D, self.t, c.filled_dev.data_ptr(), c.max_len,
                                              c.Kc.shape[2], c.Kb.shape[2], c.bc, c.stride, c.bn, L.dtype_code(c.K.dtype),
                                              L.stream_ptr()), "nsa_cache_append_dev")
+            if self._ask_split is None:
+                out = _step(self.q, c, self.gate_logits, self.scale, c.filled_dev)
+                if out is not None:
+                    return out
             Qb = ops.pool_mean(self.q, bm, bm)
             shared = bool(_cfg(cfg, "select_per_group", False))
             nq = Qb.shape[2]
