@@ -180,19 +180,12 @@ int nsa_attention_fwd(const nsa_fwd_args* args, nsa_stream_t stream) {
     return attention_fwd_tc5(*args, (cudaStream_t)stream);
   }
   if (args->engine == NSA_ENGINE_AUTO && tc5) {
-    // One block list per query head makes the tcgen05 kernel stage the union of four lists for 256 rows of
-    // which 64 use each block; measured, a selected-only launch at D=64 is then faster on the generic
-    // kernel (0.99 ms against 1.90 ms at B=2, T=32768, Hq=12, Hkv=1), everything else on tcgen05.
-    const bool sel_only_per_head = !args->fused && args->branches == NSA_BRANCH_SELECTED && args->Hi == args->H && args->D == 64 &&
-                                   args->kv_dtype == args->q_dtype;
-    // Multi-head attention (one KV head per query head) at D=64 with its per-head lists: a tcgen05 work item is then
-    // four query blocks of one head, whose four lists it merges and masks, so three quarters of the selected
-    // branch's MMA work is masked out; measured at B=1, T=65536, H=Hkv=16 the fused forward takes 3.05 ms on the
-    // generic kernel against 3.78 ms (equal at T=4096).
-    const bool mha_fused_d64 = args->fused && args->D == 64 && args->H == args->Hkv && (args->branches & NSA_BRANCH_SELECTED) &&
-                               is16(args->q_dtype) && args->kv_dtype == args->q_dtype && args->accumulate == 0 &&
-                               args->lse == nullptr && args->dyn_len == nullptr && args->nsplit <= 1;
-    if (!sel_only_per_head && !mha_fused_d64) return attention_fwd_tc5(*args, (cudaStream_t)stream);
+    // fp8 storage with one block list per query head, selected branch alone at D=64: the tcgen05 kernel stages the union of
+    // four lists for 256 rows of which 64 use each block, and the generic kernel is faster (0.99 against 1.90 ms at B=2,
+    // T=32768, Hq=12, Hkv=1).  16-bit storage walks the four lists side by side instead (attention_fwd_tc5).
+    const bool sel8_per_head = !args->fused && args->branches == NSA_BRANCH_SELECTED && args->Hi == args->H && args->D == 64 &&
+                               is8(args->q_dtype) && args->kv_dtype == args->q_dtype;
+    if (!sel8_per_head) return attention_fwd_tc5(*args, (cudaStream_t)stream);
   }
   NSA_REQUIRE(args->dyn_len == nullptr, NSA_ERR_UNSUPPORTED, "attention forward: a device-resident length needs the tcgen05 kernel");
   NSA_REQUIRE(args->kv_dtype == args->q_dtype, NSA_ERR_UNSUPPORTED, "attention forward: bf16 K/V beside an fp8 Q need the tcgen05 kernel");

@@ -81,12 +81,12 @@ __device__ __forceinline__ float row_max_raw(const uint32_t (&sv)[4][32], int nc
   return fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
 }
 
-// P = exp2(S * sl2 - m_ref) for 32 columns of a row without masked entries, as 16 packed 16-bit pairs; the row sums
-// go to the packed accumulators.  Of every 8 pairs, 3 are evaluated by the polynomial on the FMA pipe and 5 by ex2 on
+// P = exp2(S * sl2 - m_ref) for 32 columns of a row without masked entries, packed to 16-bit pairs in s[0..15]; the row
+// sums go to the packed accumulators.  Of every 8 pairs, 3 are evaluated by the polynomial on the FMA pipe and 5 by ex2 on
 // the special-function unit: alone, a warp's sweep of 128 columns is bound by that unit (1024 of 1190 clocks); mixed
 // this way it measured 947 clocks, and 2040 instead of 2410 with two warps sharing a scheduler.
 template <typename T>
-__device__ __forceinline__ void exp_group_mixed(const uint32_t (&s)[32], f32x2 SL, f32x2 NM, f32x2& sa, f32x2& sb, uint32_t (&pk)[16]) {
+__device__ __forceinline__ void exp_group_mixed(uint32_t (&s)[32], f32x2 SL, f32x2 NM, f32x2& sa, f32x2& sb) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const f32x2 x = fma2(mk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), SL, NM);
@@ -101,7 +101,7 @@ __device__ __forceinline__ void exp_group_mixed(const uint32_t (&s)[32], f32x2 S
     }
     const f32x2 pp = mk2(p0, p1);
     if (i & 1) sb = add2(sb, pp); else sa = add2(sa, pp);
-    pk[i] = Elem<T>::pack(p0, p1);
+    s[i] = Elem<T>::pack(p0, p1);
   }
 }
 
@@ -149,13 +149,24 @@ enum { B_QFULL = 0, B_KFULL = 1, B_KEMPTY = 3, B_VFULL = 5, B_VEMPTY = 7, B_SFUL
 // SPLIT: decoding-sized launches (few work items, long key ranges).  nsplit thread blocks share a work item; block s
 // takes tiles [nt*s/nsplit, nt*(s+1)/nsplit) of each branch and leaves (unnormalised O, m, l) per branch and row
 // in p.part; nsa_split_combine_kernel merges them and applies the gates.
-template <int D, int FMT, bool IN8, bool SPLIT>
+//
+// OWN (D = 64, one block list per query head): the four row groups of an item share no list.  Merged and masked, 3 of 4
+// (row, key) pairs of the selected branch were computed for nothing, and multi-head attention ran on the mma.sync kernel
+// instead (T=16384, 16 heads of their own keys, D=64: 591 us; this way 401).  A step of the selected branch takes the next
+// listed block of EACH group: a ring slot holds four 64-key chunks, MMA tile X multiplies its 128 rows with the two chunks of
+// its own two groups, a softmax thread reads only its group's 64 columns of S, and the other group's 64 columns of P are zero,
+// so one N = 64 P V over both chunks adds to every row what its own chunk gives.  The tensor pipe does each product twice
+// over, which costs nothing here: it is busy 20 % of the time, the softmax warps' serial sweep is what a step takes.
+// The running gated sum is held in fp32 in shared memory: D = 64 leaves the room, and the result is rounded once.
+template <int D, int FMT, bool IN8, bool SPLIT, bool OWN = false>
 __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_constant__ Tc5Params p) {
   using T = typename std::conditional<FMT == 1, __nv_bfloat16, __half>::type;
   constexpr int DH = D / 64;                    // 64-element (128-byte) halves of a row
   constexpr int QTILE = DH * 128 * 128;         // bytes of one 128-row Q tile
   constexpr int KVTILE = DH * 128 * 128;        // bytes of one 128-key K or V tile
   constexpr int DHSTRIDE = 128 * 128;           // bytes between the halves
+  static_assert(!OWN || (D == 64 && !IN8 && !SPLIT), "own lists: D = 64, 16-bit storage, unsplit");
+  constexpr int KVSLOT = OWN ? 2 * KVTILE : KVTILE;   // bytes of a ring slot: own lists stage one tile per MMA tile
   // D = 64 leaves 64 TMEM columns per tile unused: P gets columns of its own there instead of aliasing S,
   // so the next tile's QK^T can be issued as soon as the softmax threads hold the S row in registers
   // (not only after PV has consumed P) -- the QK -> softmax -> PV chain of a tile is broken.
@@ -166,7 +177,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sQ = smem_u32(smem);
   const uint32_t sK = sQ + 2 * QTILE;
-  const uint32_t sV = sK + 2 * KVTILE;
+  const uint32_t sV = sK + 2 * KVSLOT;
   // fp8 storage only: two staging buffers of 128 rows x D bytes (plain row-major), filled by TMA and turned
   // into the swizzled 16-bit tiles above by warps 2 (K side) and 3 (V side); Q goes through them first
   constexpr int STG = 128 * D;
@@ -175,6 +186,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
   __shared__ int sel_list[T5_MAX_ENT];            // selected branch: key blocks to visit ...
   __shared__ unsigned char sel_mask[T5_MAX_ENT];  // ... and the row groups that listed each of them
   __shared__ int sel_n;
+  __shared__ int sel_cnt[4];                      // own lists: entries of each row group, at sel_list[group * T5_MAX_SEL ..]
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
 
@@ -256,7 +268,33 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
     // 4 lists are merged: a block listed by several groups is staged once and masked per group; a block
     // listed p times by one group is visited p times (the reference counts duplicates twice).
     int n = 0;
-    if (a.branches & NSA_BRANCH_SELECTED) {
+    if constexpr (OWN) {
+      if (a.branches & NSA_BRANCH_SELECTED) {
+        int blk[4][T5_MAX_SEL / 32];
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+#pragma unroll
+          for (int c = 0; c < T5_MAX_SEL / 32; ++c) {
+            const int qb = grp_qb(g), sl = c * 32 + lane;
+            blk[g][c] = qb < a.nq && sl < a.top_k ? a.idx[(((size_t)b * a.Hi + grp_head(g)) * a.nq + qb) * a.top_k + sl] : -1;
+          }
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          const int last_pos = min(grp_qb(g) * 64 + 64, a.Tq) - 1 + OFFSET();
+          int cnt = 0;
+#pragma unroll
+          for (int c = 0; c < T5_MAX_SEL / 32; ++c) {
+            const int v = blk[g][c];
+            const bool take = v >= 0 && v < SEL_LIMIT() / 64 && (!a.causal || (long long)v * 64 <= last_pos);
+            const unsigned bal = __ballot_sync(0xffffffffu, take);
+            if (take) sel_list[g * T5_MAX_SEL + cnt + __popc(bal & ((1u << lane) - 1))] = v;
+            cnt += __popc(bal);
+          }
+          if (lane == 0) sel_cnt[g] = cnt;
+          n = max(n, 2 * cnt);                              // a step is two chunks per MMA tile
+        }
+      }
+    } else if (a.branches & NSA_BRANCH_SELECTED) {
       const bool shared = a.Hi != a.H && GH == 4;
       const int ngrp = shared ? 1 : 4;
       const int n_ent = ngrp * a.top_k;
@@ -411,6 +449,32 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
             __syncwarp();
             continue;
           }
+          if constexpr (OWN) {
+            if (br == 1) {
+              // the next listed block of each row group; a group whose list has ended gets block 0, masked out by its rows
+              int j0[4];
+#pragma unroll
+              for (int g = 0; g < 4; ++g) j0[g] = t < sel_cnt[g] ? sel_list[g * T5_MAX_SEL + t] * 64 : 0;
+              ok = __all_sync(0xffffffffu, mbar_wait(bar(B_KEMPTY + s), ph ^ 1, &abort_flag));
+              if (!ok) { fail_id = B_KEMPTY + s + 1; break; }
+              if (leader) {
+                mbar_expect_tx(bar(B_KFULL + s), KVSLOT);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) tma_load_3d(sK + s * KVSLOT + g * 8192, mk, bar(B_KFULL + s), 0, j0[g], kv_slab);
+              }
+              last_k_it = it;
+              ok = __all_sync(0xffffffffu, mbar_wait(bar(B_VEMPTY + s), ph ^ 1, &abort_flag));
+              if (!ok) { fail_id = B_VEMPTY + s + 1; break; }
+              if (leader) {
+                mbar_expect_tx(bar(B_VFULL + s), KVSLOT);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) tma_load_3d(sV + s * KVSLOT + g * 8192, mv, bar(B_VFULL + s), 0, j0[g], kv_slab);
+              }
+              last_v_it = it;
+              __syncwarp();
+              continue;
+            }
+          }
           const uint32_t bytes = (uint32_t)tl.nch * 64 * D * 2;
           ok = __all_sync(0xffffffffu, mbar_wait(bar(B_KEMPTY + s), ph ^ 1, &abort_flag));
           if (!ok) { fail_id = B_KEMPTY + s + 1; break; }
@@ -418,7 +482,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
             mbar_expect_tx(bar(B_KFULL + s), bytes);
             for (int c = 0; c < tl.nch; ++c)
               for (int dh = 0; dh < DH; ++dh)
-                tma_load_3d(sK + s * KVTILE + dh * DHSTRIDE + c * 8192, mk, bar(B_KFULL + s), dh * 64, tl.j0[c], kv_slab);
+                tma_load_3d(sK + s * KVSLOT + dh * DHSTRIDE + c * 8192, mk, bar(B_KFULL + s), dh * 64, tl.j0[c], kv_slab);
           }
           last_k_it = it;
           ok = __all_sync(0xffffffffu, mbar_wait(bar(B_VEMPTY + s), ph ^ 1, &abort_flag));
@@ -427,7 +491,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
             mbar_expect_tx(bar(B_VFULL + s), bytes);
             for (int c = 0; c < tl.nch; ++c)
               for (int dh = 0; dh < DH; ++dh)
-                tma_load_3d(sV + s * KVTILE + dh * DHSTRIDE + c * 8192, mv, bar(B_VFULL + s), dh * 64, tl.j0[c], kv_slab);
+                tma_load_3d(sV + s * KVSLOT + dh * DHSTRIDE + c * 8192, mv, bar(B_VFULL + s), dh * 64, tl.j0[c], kv_slab);
           }
           last_v_it = it;
           __syncwarp();
@@ -452,8 +516,8 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
       for (int br = 0; br < 3; ++br) { nt_of[br] = tend(br) - tbeg(br); total_tiles += nt_of[br]; }
       // descriptor bases: the low word carries the address field, so "+ (bytes >> 4)" moves the start
       const uint64_t dQ[2] = {smem_desc_sw128(sQ, 16, 1024), smem_desc_sw128(sQ + QTILE, 16, 1024)};
-      const uint64_t dK[2] = {smem_desc_sw128(sK, 16, 1024), smem_desc_sw128(sK + KVTILE, 16, 1024)};
-      const uint64_t dV[2] = {smem_desc_sw128(sV, DHSTRIDE, 1024), smem_desc_sw128(sV + KVTILE, DHSTRIDE, 1024)};
+      const uint64_t dK[2] = {smem_desc_sw128(sK, 16, 1024), smem_desc_sw128(sK + KVSLOT, 16, 1024)};
+      const uint64_t dV[2] = {smem_desc_sw128(sV, DHSTRIDE, 1024), smem_desc_sw128(sV + KVSLOT, DHSTRIDE, 1024)};
       const uint32_t tSx[2] = {tmem, tmem + 128}, tOx[2] = {tmem + 256, tmem + 384};
       const uint32_t tPx[2] = {EARLY ? tmem + 320 : tmem, EARLY ? tmem + 448 : tmem + 128};
 
@@ -471,12 +535,13 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
           tc_fence_after();
         }
         const uint32_t idesc = nch == 2 ? IDESC_QK2 : IDESC_QK1;
+        const uint64_t dKs = dK[s] + ((OWN && q_br == 1) ? X * (KVTILE >> 4) : 0);   // own lists: tile X's own chunks
         if (leader) {
 #pragma unroll
           for (int ks = 0; ks < D / 16; ++ks) {
             const uint32_t off = (uint32_t)(((ks >> 2) * DHSTRIDE + (ks & 3) * 32) >> 4);
-            if (ks == 0) mma_ss(tSx[X], dQ[X] + off, dK[s] + off, idesc, 0u);
-            else mma_ss(tSx[X], dQ[X] + off, dK[s] + off, idesc, 1u);
+            if (ks == 0) mma_ss(tSx[X], dQ[X] + off, dKs + off, idesc, 0u);
+            else mma_ss(tSx[X], dQ[X] + off, dKs + off, idesc, 1u);
           }
           tc_commit(bar(B_SFULL + X));
           if (X == 1) tc_commit(bar(B_KEMPTY + s));
@@ -508,16 +573,17 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
 #pragma unroll
         for (int X = 0; X < 2; ++X) {
           if (!ok) break;
+          const uint64_t dVs = dV[s] + ((OWN && p_br == 1) ? X * (KVTILE >> 4) : 0);
           if constexpr (!EARLY) {
             // first 64 keys of P V as soon as that half of P is written
             ok = __all_sync(0xffffffffu, mbar_wait_spin(bar(B_PHALF + X), it & 1, &abort_flag));
             if (!ok) { fail_id = B_PHALF + X + 1; break; }
             tc_fence_after();
             if (leader) {
-              if (fresh) mma_ts(tOx[X], tPx[X], dV[s], IDESC_PV, 0u);
-              else mma_ts(tOx[X], tPx[X], dV[s], IDESC_PV, 1u);
+              if (fresh) mma_ts(tOx[X], tPx[X], dVs, IDESC_PV, 0u);
+              else mma_ts(tOx[X], tPx[X], dVs, IDESC_PV, 1u);
 #pragma unroll
-              for (int kk = 1; kk < 4; ++kk) mma_ts(tOx[X], tPx[X] + kk * 8, dV[s] + kk * 128, IDESC_PV, 1u);
+              for (int kk = 1; kk < 4; ++kk) mma_ts(tOx[X], tPx[X] + kk * 8, dVs + kk * 128, IDESC_PV, 1u);
             }
             __syncwarp();
           }
@@ -526,14 +592,14 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
           tc_fence_after();
           if (leader) {
             if constexpr (EARLY) {
-              if (fresh) mma_ts(tOx[X], tPx[X], dV[s], IDESC_PV, 0u);
-              else mma_ts(tOx[X], tPx[X], dV[s], IDESC_PV, 1u);
+              if (fresh) mma_ts(tOx[X], tPx[X], dVs, IDESC_PV, 0u);
+              else mma_ts(tOx[X], tPx[X], dVs, IDESC_PV, 1u);
 #pragma unroll
-              for (int kk = 1; kk < 4; ++kk) mma_ts(tOx[X], tPx[X] + kk * 8, dV[s] + kk * 128, IDESC_PV, 1u);
+              for (int kk = 1; kk < 4; ++kk) mma_ts(tOx[X], tPx[X] + kk * 8, dVs + kk * 128, IDESC_PV, 1u);
             }
             if (nch == 2) {
 #pragma unroll
-              for (int kk = 4; kk < 8; ++kk) mma_ts(tOx[X], tPx[X] + kk * 8, dV[s] + kk * 128, IDESC_PV, 1u);
+              for (int kk = 4; kk < 8; ++kk) mma_ts(tOx[X], tPx[X] + kk * 8, dVs + kk * 128, IDESC_PV, 1u);
             }
             tc_commit(bar(B_PVDONE + X));
             if (X == 1) tc_commit(bar(B_VEMPTY + s));
@@ -653,7 +719,8 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
     // loads and stores were 12 % of the kernel.  Only the item's last branch writes these columns out; the values
     // are the same, rounded to 16 bits at every branch end.  At D = 64 that is the whole row.
     const bool keep = !SPLIT && !IN8 && p.psum != 0;
-    unsigned char* prow_s = smem + 2 * QTILE + 4 * KVTILE + (size_t)(X * 128 + r) * 128;
+    // (own lists: the whole row in fp32, 256 bytes, and rounded once)
+    unsigned char* prow_s = smem + 2 * QTILE + 4 * KVSLOT + (size_t)(X * 128 + r) * (OWN ? 256 : 128);
     bool kept = false;                                   // the shared-memory columns hold a partial sum
     // The item's LAST branch end (every column goes to the output row) stages its 16-bit values in shared memory -- columns
     // 0..63 where the partial sums lay, 64..127 in the Q tiles' area, which no MMA reads any more -- as two boxes of 32 rows
@@ -682,17 +749,38 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
       int lo, hi;
       bounds(br, qi, row_ok, lo, hi);
       float m_used = -INFINITY, l = 0.f;
+      const bool own = OWN && br == 1;
+      const int half = own ? quarter >> 1 : 0;             // own lists: this row's 64 columns of S and P
+      if constexpr (OWN) {
+        if (own) {                                         // the other group's columns of P stay zero for the whole branch
+          uint32_t z[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) z[i] = 0u;
+          tmem_st16(tP + (half ^ 1) * 32, z);
+          tmem_st16(tP + (half ^ 1) * 32 + 16, z);
+        }
+      }
       const float sl2 = p.scale_log2[br];
 #pragma unroll 1
       for (int t = tbeg(br); t < tend(br) && ok; ++t, ++it) {
-        const Tile tl = get_tile(br, t);
+        Tile tl = get_tile(br, t);
+        if constexpr (OWN) {
+          if (own) {
+            const bool listed = t < sel_cnt[rg];
+            const int blk = listed ? sel_list[rg * T5_MAX_SEL + t] : 0;
+            tl.nch = 1;
+            tl.j0[0] = blk * 64;
+            tl.jlim[0] = min(blk * 64 + 64, SEL_LIMIT());
+            tl.mask[0] = listed ? 0xF : 0;
+          }
+        }
         ok = __all_sync(0xffffffffu, mbar_wait(bar(B_SFULL + X), it & 1, &abort_flag));
         if (!ok) { fail_id = B_SFULL + X + 1; break; }
         tc_fence_after();
         // the whole S row of the tile: 64*nch columns, one wait
         uint32_t sv[4][32];
-        tmem_ld32(tS, sv[0]);
-        tmem_ld32(tS + 32, sv[1]);
+        tmem_ld32(tS + half * 64, sv[0]);
+        tmem_ld32(tS + half * 64 + 32, sv[1]);
         if (tl.nch == 2) { tmem_ld32(tS + 64, sv[2]); tmem_ld32(tS + 96, sv[3]); }
         tc_wait_ld();
         if constexpr (EARLY) {                             // S is in registers: the MMA warp may overwrite it
@@ -740,13 +828,6 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
           m_used = m_new;
         }
         const float m_ref = m_used == -INFINITY ? 0.f : m_used;
-        if constexpr (EARLY) {
-          if (it > 0) {                                    // P's columns are free once the previous PV has read them
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(B_PVDONE + X), (it - 1) & 1, &abort_flag));
-            if (!ok) { fail_id = B_PVDONE + X + 1; break; }
-            tc_fence_after();
-          }
-        }
         // P = exp2(S*scale - m_ref) as 16-bit (-inf -> 0)
         if (use_poly) {
           const f32x2 SL = mk2(sl2, sl2), NM = mk2(-m_ref, -m_ref);
@@ -754,9 +835,8 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
             if (g < 2 * tl.nch) {
-              uint32_t pk[16];
-              exp_group_mixed<T>(sv[g], SL, NM, sa, sb, pk);
-              tmem_st16(tP + g * 16, pk);
+              exp_group_mixed<T>(sv[g], SL, NM, sa, sb);
+              if constexpr (!EARLY) tmem_st16(tP + half * 32 + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
             }
             if (!EARLY && g == 1) { tc_wait_st(); tc_fence_before(); mbar_arrive(bar(B_PHALF + X)); }
           }
@@ -768,21 +848,32 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
             if (g < 2 * tl.nch) {
-              uint32_t pk[16];
 #pragma unroll
               for (int i = 0; i < 16; ++i) {
                 const float p0 = ex2(fmaf(__uint_as_float(sv[g][2 * i]), sl2, -m_ref));
                 const float p1 = ex2(fmaf(__uint_as_float(sv[g][2 * i + 1]), sl2, -m_ref));
                 if (i & 1) { psum2 += p0; psum3 += p1; } else { psum0 += p0; psum1 += p1; }
-                pk[i] = Elem<T>::pack(p0, p1);
+                sv[g][i] = Elem<T>::pack(p0, p1);
               }
-              tmem_st16(tP + g * 16, pk);
+              if constexpr (!EARLY) tmem_st16(tP + half * 32 + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
             }
             if (!EARLY && g == 1) { tc_wait_st(); tc_fence_before(); mbar_arrive(bar(B_PHALF + X)); }
           }
           psum0 += psum2;
           psum1 += psum3;
           l += psum0 + psum1;
+        }
+        if constexpr (EARLY) {
+          // P's columns are free once the previous PV has read them: waited for here, with the exponentials done and packed, so
+          // that PV runs under this tile's sweep and not before it (D=64, 64 heads over 4, T=16384: -2 %)
+          if (it > 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(B_PVDONE + X), (it - 1) & 1, &abort_flag));
+            if (!ok) { fail_id = B_PVDONE + X + 1; break; }
+            tc_fence_after();
+          }
+#pragma unroll
+          for (int g = 0; g < 4; ++g)
+            if (g < 2 * tl.nch) tmem_st16(tP + half * 32 + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
         }
         tc_wait_st();
         tc_fence_before();
@@ -793,7 +884,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
       // The running gated sum of the earlier branches is read back from the output row NOW, before that wait: the
       // loads fly while the last PV executes instead of costing a memory round trip per 64 bytes afterwards.
       uint4 prevv[D / 8];
-      if constexpr (!SPLIT) {
+      if constexpr (!SPLIT && !OWN) {
 #pragma unroll
         for (int c = 0; c < D / 8; ++c) {
           if (c < 8 && kept) prevv[c] = *reinterpret_cast<const uint4*>(prow_s + ((c ^ (r & 7)) << 4));
@@ -823,6 +914,42 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
       const bool has = l > 0.f;
       const float coef = has ? (a.fused ? gate[br] : 1.f) * p.out_scale[br] / l : 0.f;
       if (a.lse != nullptr) lse_out = has ? m_used * kLn2 + __logf(l) : -INFINITY;   // one branch per launch when lse is asked for
+      if constexpr (OWN) {
+#pragma unroll
+        for (int g = 0; g < D / 32; ++g) {
+          uint32_t v[32];
+          tmem_ld32(tO + g * 32, v);
+          tc_wait_ld();
+          if (row_ok) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              float acc[8];
+              float4* q0 = reinterpret_cast<float4*>(prow_s + (((g * 8 + 2 * c) ^ (r & 7)) << 4));
+              float4* q1 = reinterpret_cast<float4*>(prow_s + (((g * 8 + 2 * c + 1) ^ (r & 7)) << 4));
+              if (kept) {
+                const float4 x = *q0, y = *q1;
+                acc[0] = x.x; acc[1] = x.y; acc[2] = x.z; acc[3] = x.w; acc[4] = y.x; acc[5] = y.y; acc[6] = y.z; acc[7] = y.w;
+              } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+              }
+#pragma unroll
+              for (int e = 0; e < 8; ++e) acc[e] = fmaf(__uint_as_float(v[8 * c + e]), coef, acc[e]);
+              if (br != last_br) {
+                *q0 = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                *q1 = make_float4(acc[4], acc[5], acc[6], acc[7]);
+              } else {
+                reinterpret_cast<uint4*>(orow)[g * 4 + c] = make_uint4(Elem<T>::pack(acc[0], acc[1]), Elem<T>::pack(acc[2], acc[3]),
+                                                                       Elem<T>::pack(acc[4], acc[5]), Elem<T>::pack(acc[6], acc[7]));
+              }
+            }
+          }
+        }
+        have_partial = true;
+        kept = br != last_br;
+        tc_fence_before();
+        continue;
+      }
 #pragma unroll
       for (int g = 0; g < D / 32; ++g) {
         uint32_t v[32];
@@ -1432,22 +1559,14 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __gri
             m_used = m_new;
           }
           const float m_ref = m_used == -INFINITY ? 0.f : m_used;
-          if constexpr (EARLY) {
-            if (it > 0) {
-              ok = __all_sync(0xffffffffu, mbar_wait(bar(B_PVDONE + X), (it - 1) & 1, &abort_flag));
-              if (!ok) { fail_id = B_PVDONE + X + 1; break; }
-              tc_fence_after();
-            }
-          }
           if (use_poly) {
             const f32x2 SL = mk2(sl2, sl2), NM = mk2(-m_ref, -m_ref);
             f32x2 sa = mk2(0.f, 0.f), sb = mk2(0.f, 0.f);
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
               if (g < 2 * tl.nch) {
-                uint32_t pk[16];
-                exp_group_mixed<T>(sv[g], SL, NM, sa, sb, pk);
-                tmem_st16(tP + g * 16, pk);
+                exp_group_mixed<T>(sv[g], SL, NM, sa, sb);
+                if constexpr (!EARLY) tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
               }
             }
             float s0, s1;
@@ -1458,20 +1577,31 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __gri
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
               if (g < 2 * tl.nch) {
-                uint32_t pk[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                   const float p0 = ex2(fmaf(__uint_as_float(sv[g][2 * i]), sl2, -m_ref));
                   const float p1 = ex2(fmaf(__uint_as_float(sv[g][2 * i + 1]), sl2, -m_ref));
                   if (i & 1) { psum2 += p0; psum3 += p1; } else { psum0 += p0; psum1 += p1; }
-                  pk[i] = Elem<T>::pack(p0, p1);
+                  sv[g][i] = Elem<T>::pack(p0, p1);
                 }
-                tmem_st16(tP + g * 16, pk);
+                if constexpr (!EARLY) tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
               }
             }
             psum0 += psum2;
             psum1 += psum3;
             l += psum0 + psum1;
+          }
+          if constexpr (EARLY) {
+            // P's columns are free once the previous PV has read them: waited for here, with the exponentials done and packed, so
+            // that PV runs under this tile's sweep and not before it (D=64, 64 heads over 4, T=16384: -2 %)
+            if (it > 0) {
+              ok = __all_sync(0xffffffffu, mbar_wait(bar(B_PVDONE + X), (it - 1) & 1, &abort_flag));
+              if (!ok) { fail_id = B_PVDONE + X + 1; break; }
+              tc_fence_after();
+            }
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+              if (g < 2 * tl.nch) tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
           }
           tc_wait_st();
           tc_fence_before();
@@ -1809,7 +1939,15 @@ int attention_fwd_tc5(const nsa_fwd_args& a, cudaStream_t st) {
   }
   const long long blocks = items * p.nsplit;
   NSA_REQUIRE(blocks > 0 && blocks < 2147483647LL, NSA_ERR_ARG, "attention forward: %lld work items do not fit a grid", blocks);
-  const size_t smem = (size_t)(2 + 2 + 2) * (a.D / 64) * 128 * 128 + (in8 ? (size_t)2 * 128 * a.D : 0) + (p.psum ? 256 * 128 : 0) + 1024;
+  // One block list per query head at D = 64: every row group walks its own list (OWN).  Against the mma.sync kernel, whole
+  // forwards of 16 heads with their own keys: T=512 52.9 against 50.6 us, 1024 73.1 / 74.3, 2048 75.6 / 94.6, 4096 129 / 164,
+  // 16384 438 / 629, 32768 890 / 1329; 16 heads over one, B=2, T=4001: 204 / 302 (four lists merged and masked: 383).
+  // Launches that add to a 16-bit partial sum, and callers that name the engine, keep the merged lists: a branch added to
+  // the rows afterwards and the same branches in one launch then give the same bits.
+  const bool own = !in8 && !split && a.D == 64 && (a.branches & NSA_BRANCH_SELECTED) && a.Hi == a.H && a.engine == NSA_ENGINE_AUTO &&
+                   a.accumulate == 0;
+  const size_t smem = own ? (size_t)(2 + 4 + 4) * 128 * 128 + 256 * 256 + 1024 :
+                      (size_t)(2 + 2 + 2) * (a.D / 64) * 128 * 128 + (in8 ? (size_t)2 * 128 * a.D : 0) + (p.psum ? 256 * 128 : 0) + 1024;
 #define NSA_TC5_LAUNCH(DD, FF, I8, SP)                                                                     \
   {                                                                                                         \
     auto fn = nsa_fwd_tc5_kernel<DD, FF, I8, SP>;                                                           \
@@ -1832,6 +1970,18 @@ int attention_fwd_tc5(const nsa_fwd_args& a, cudaStream_t st) {
     else if (fmt == 1) NSA_TC5_COMBINE(__nv_bfloat16, 64);
     else NSA_TC5_COMBINE(__half, 64);
 #undef NSA_TC5_COMBINE
+  }
+  if (own) {
+#define NSA_TC5_LAUNCH_OWN(FF)                                                                              \
+  {                                                                                                         \
+    auto fn = nsa_fwd_tc5_kernel<64, FF, false, false, true>;                                               \
+    NSA_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));         \
+    fn<<<(unsigned)blocks, T5_THREADS, smem, st>>>(p);                                                     \
+  }
+    p.poly = 0;                        // every exponential on ex2, as on the mma.sync kernel
+    if (fmt == 1) NSA_TC5_LAUNCH_OWN(1) else NSA_TC5_LAUNCH_OWN(0)
+#undef NSA_TC5_LAUNCH_OWN
+    return launch_status("attn_fwd_tc5 (own lists)");
   }
   const int n_br = ((a.branches >> 0) & 1) + ((a.branches >> 1) & 1) + ((a.branches >> 2) & 1);
   if (!in8 && (tc5_persistent_mode() == 1 || (tc5_persistent_mode() == -1 && n_br == 1))) {

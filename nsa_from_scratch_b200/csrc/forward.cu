@@ -22,8 +22,8 @@ static bool fp8(int dt) { return dt == NSA_FP8_E4M3 || dt == NSA_FP8_E5M2; }
 
 struct ForwardPlan {
   int Nc, nq, nk, k_sel, Hi;
-  bool select, dequant;
-  size_t o_qb, o_kb, o_kc, o_vc, o_idx, o_k16, o_v16, total;
+  bool select, dequant, dequant_q;
+  size_t o_qb, o_kb, o_kc, o_vc, o_idx, o_k16, o_v16, o_q16, total;
 };
 
 static int forward_plan(const nsa_forward_args& f, ForwardPlan& pl) {
@@ -48,6 +48,8 @@ static int forward_plan(const nsa_forward_args& f, ForwardPlan& pl) {
   a.bm = f.bm; a.bn = f.bn; a.top_k = pl.k_sel; a.Nc = pl.Nc;
   a.branches = NSA_BRANCH_COMPRESSED | NSA_BRANCH_SELECTED | NSA_BRANCH_SLIDING;
   pl.dequant = fp8(f.q_dtype) && f.engine != NSA_ENGINE_GENERIC && attention_fwd_tc5_supports(a);
+  // one list per query head at D = 64: Q as well, for the kernel whose row groups walk their own lists (16-bit storage)
+  pl.dequant_q = pl.dequant && f.D == 64 && pl.Hi == f.H && f.engine == NSA_ENGINE_AUTO;
   auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
   const size_t row = (size_t)f.D * 2, kv = (size_t)f.B * f.Hkv;
   size_t o = 0;
@@ -58,6 +60,7 @@ static int forward_plan(const nsa_forward_args& f, ForwardPlan& pl) {
   pl.o_idx = o; if (pl.select) o = up(o + (size_t)f.B * pl.Hi * pl.nq * pl.k_sel * 4);
   pl.o_k16 = o; if (pl.dequant) o = up(o + kv * f.Tk * row);
   pl.o_v16 = o; if (pl.dequant) o = up(o + kv * f.Tk * row);
+  pl.o_q16 = o; if (pl.dequant_q) o = up(o + (size_t)f.B * f.H * f.Tq * row);
   pl.total = o < 256 ? 256 : o;
   return NSA_OK;
 }
@@ -131,6 +134,12 @@ int nsa_forward(const nsa_forward_args* fa, nsa_stream_t stream) {
     V = ws + pl.o_v16;
   }
   nsa_fwd_args a = attention_args(f, pl, K, V, ws + pl.o_kc, ws + pl.o_vc, idx);
+  if (pl.dequant_q) {
+    if ((rc = fp8_dequantize(f.Q, ws + pl.o_q16, (long long)BH * f.Tq * f.D, f.q_dtype, f.q_scale, st)) != NSA_OK) return rc;
+    a.Q = ws + pl.o_q16;
+    a.q_dtype = NSA_BF16;
+    a.q_scale = a.k_scale = a.v_scale = 1.f;
+  }
   a.out = f.out; a.gates = f.gates; a.gate_dtype = f.gate_dtype;
   a.branches = NSA_BRANCH_COMPRESSED | NSA_BRANCH_SELECTED | NSA_BRANCH_SLIDING;
   a.fused = 1;

@@ -201,7 +201,8 @@ def attention_fwd(
     `accumulate_into`: the output of an earlier fused launch (other branches); this launch adds its branches to it
     and returns the same tensor.  `fused_lse`: a fused launch of ONE branch also returns that branch's lse.
     `dequant_kv` (fp8 inputs): True/False forces / forbids the one-off dequantisation of K and V in front of the
-    launch; None decides by kernel (see below).  The results are identical either way."""
+    launch; None decides by kernel (see below).  The results are identical either way.  (One list per head at D=64:
+    the flag has no say, that kernel takes 16-bit tensors.)"""
     _need_cuda(Q, K, V)
     B, H, Tq, D = Q.shape
     Hkv, Tk = K.shape[1], K.shape[2]
@@ -217,10 +218,16 @@ def attention_fwd(
         # The tcgen05 kernel takes an fp8 Q with bf16 K/V: a K/V tile is used by every query block that attends it,
         # so K and V are dequantised ONCE here (with GQA they are a small fraction of Q) instead of once per use
         # inside the kernel, where the conversion, not the tensor pipe, set the pace; Q's tiles are used once and
-        # stay fp8 in HBM.  A selected-only launch with one list per head at D=64 runs on the generic kernel.
-        per_head_sel = (not fused and branches == L.BRANCH_SELECTED and idx is not None and idx.shape[1] == H and D == 64
-                        and eng == L.ENGINE_AUTO)
-        if (not per_head_sel) if dequant_kv is None else dequant_kv:
+        # stay fp8 in HBM.  With one list per head at D=64 Q is dequantised too: the kernel whose row groups walk their
+        # own lists takes 16-bit storage; where that one does not apply, a selected-only launch runs on the generic kernel.
+        per_head = D == 64 and idx is not None and (branches & L.BRANCH_SELECTED) != 0 and idx.shape[1] == H
+        own_lists = (per_head and eng == L.ENGINE_AUTO and accumulate_into is None and nsplit <= 1 and dyn_len is None
+                     and bm == bn == 64 and idx.shape[3] <= 64 and min(scale, q_scale, k_scale, v_scale) > 0)
+        per_head_sel = per_head and not own_lists and not fused and branches == L.BRANCH_SELECTED and eng == L.ENGINE_AUTO
+        if own_lists:
+            Q, K, V = fp8_dequantize(Q, q_scale), fp8_dequantize(K, k_scale), fp8_dequantize(V, v_scale)
+            q_scale = k_scale = v_scale = 1.0
+        elif (not per_head_sel) if dequant_kv is None else dequant_kv:
             K, V = fp8_dequantize(K, k_scale), fp8_dequantize(V, v_scale)
     out_dtype = torch.bfloat16 if Q.dtype in _8 else Q.dtype
     if accumulate_into is not None:
