@@ -19,6 +19,11 @@
 //               row sum, P as 16-bit back into TMEM; at the end of a branch they read O, apply
 //               gate/l and add it into the output row (the row itself holds the running gated sum)
 // TMEM columns: S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [384,384+D).
+// The softmax loop is laid out for instruction fetch: its unmasked path is one straight line (a wait that is over, the
+// load, the maximum, the exponentials by one route for all 128 columns), and masks, rescales and the all-ex2 route
+// stand behind branches marked unlikely.  Masking chunk by chunk and choosing per 32 columns in line, with the tile's description rebuilt
+// by a three-way branch, the same work had its warps out of instructions for a third of their time (three warps per scheduler hide
+// no fetch): 64 heads over 4, T=16384: D=128 1594 -> 1496 us, D=64 1434 -> 1214 us.
 // Tile X's chain QK -> softmax -> PV is serial; the tensor pipe stays busy because the other
 // tile's MMAs run in the gaps.  Every mbarrier wait is bounded; a wait that gives up raises a
 // block-wide abort flag, sets the device status word and the block still frees its TMEM.
@@ -27,6 +32,7 @@
 
 #include <cudaTypedefs.h>
 #include <stdlib.h>
+#include <type_traits>
 
 namespace nsa {
 
@@ -65,33 +71,38 @@ struct Tile {
   int mask[2];   // which of the 4 row groups attend the chunk (selected branch; 0xF otherwise)
 };
 
-// Row maximum (raw scores) of the 64 * nch columns a softmax thread holds: four chains of 3-input max.
-__device__ __forceinline__ float row_max_raw(const uint32_t (&sv)[4][32], int nch) {
+// Row maximum (raw scores) of the 32 * NG columns a softmax thread holds: four chains of 3-input max.
+template <int NG>
+__device__ __forceinline__ float row_max_raw(const uint32_t (&sv)[4][32]) {
   float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-  for (int g = 0; g < 2; ++g)
+  for (int g = 0; g < NG; ++g)
 #pragma unroll
     for (int i = 0; i < 32; i += 2) m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], __uint_as_float(sv[g][i]), __uint_as_float(sv[g][i + 1]));
-  if (nch == 2) {
-#pragma unroll
-    for (int g = 2; g < 4; ++g)
-#pragma unroll
-      for (int i = 0; i < 32; i += 2) m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], __uint_as_float(sv[g][i]), __uint_as_float(sv[g][i + 1]));
-  }
   return fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
 }
 
-// P = exp2(S * sl2 - m_ref) for 32 columns of a row without masked entries, packed to 16-bit pairs in s[0..15]; the row
-// sums go to the packed accumulators.  Of every 8 pairs, 3 are evaluated by the polynomial on the FMA pipe and 5 by ex2 on
-// the special-function unit: alone, a warp's sweep of 128 columns is bound by that unit (1024 of 1190 clocks); mixed
-// this way it measured 947 clocks, and 2040 instead of 2410 with two warps sharing a scheduler.
-template <typename T>
-__device__ __forceinline__ void exp_group_mixed(uint32_t (&s)[32], f32x2 SL, f32x2 NM, f32x2& sa, f32x2& sb) {
+// Columns c0..c0+31 of a softmax thread's row: those outside vlo..vhi become -inf (one bit per column and a select; two
+// compares and a select per column cost as much as the exponentials).
+__device__ __forceinline__ void mask_group(uint32_t (&s)[32], int c0, int vlo, int vhi) {
+  const int lo = vlo - c0, hi = vhi - c0;
+  const uint32_t keep = (hi < 0 || lo > 31) ? 0u : ((0xffffffffu << max(lo, 0)) & (0xffffffffu >> (31 - min(hi, 31))));
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (!((keep >> i) & 1u)) s[i] = 0xff800000u;   // -inf
+}
+
+// P = exp2(S * sl2 - m_ref) for 32 columns of a row, packed to 16-bit pairs in s[0..15]; the row sums go to the packed
+// accumulators.  POLY (columns without masked entries): of every 8 pairs, 3 are evaluated by the polynomial on the FMA pipe
+// and 5 by ex2 on the special-function unit: alone, a warp's sweep of 128 columns is bound by that unit (1024 of 1190
+// clocks); mixed this way it measured 947 clocks, and 2040 instead of 2410 with two warps sharing a scheduler.
+template <typename T, bool POLY>
+__device__ __forceinline__ void exp_group(uint32_t (&s)[32], f32x2 SL, f32x2 NM, f32x2& sa, f32x2& sb) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const f32x2 x = fma2(mk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), SL, NM);
     float p0, p1;
-    if ((i & 7) < 3) {
+    if (POLY && (i & 7) < 3) {
       exp2_poly_pair(x, p0, p1);
     } else {
       float x0, x1;
@@ -152,7 +163,7 @@ enum { B_QFULL = 0, B_KFULL = 1, B_KEMPTY = 3, B_VFULL = 5, B_VEMPTY = 7, B_SFUL
 //
 // OWN (D = 64, one block list per query head): the four row groups of an item share no list.  Merged and masked, 3 of 4
 // (row, key) pairs of the selected branch were computed for nothing, and multi-head attention ran on the mma.sync kernel
-// instead (T=16384, 16 heads of their own keys, D=64: 591 us; this way 401).  A step of the selected branch takes the next
+// instead (T=16384, 16 heads of their own keys, D=64: 591 us; this way 350).  A step of the selected branch takes the next
 // listed block of EACH group: a ring slot holds four 64-key chunks, MMA tile X multiplies its 128 rows with the two chunks of
 // its own two groups, a softmax thread reads only its group's 64 columns of S, and the other group's 64 columns of P are zero,
 // so one N = 64 P V over both chunks adds to every row what its own chunk gives.  The tensor pipe does each product twice
@@ -763,51 +774,51 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
       const float sl2 = p.scale_log2[br];
 #pragma unroll 1
       for (int t = tbeg(br); t < tend(br) && ok; ++t, ++it) {
-        Tile tl = get_tile(br, t);
-        if constexpr (OWN) {
-          if (own) {
-            const bool listed = t < sel_cnt[rg];
-            const int blk = listed ? sel_list[rg * T5_MAX_SEL + t] : 0;
-            tl.nch = 1;
-            tl.j0[0] = blk * 64;
-            tl.jlim[0] = min(blk * 64 + 64, SEL_LIMIT());
-            tl.mask[0] = listed ? 0xF : 0;
-          }
+        // columns a0..b0 of the tile's first 64 keys and a1..b1 of its second 64 count for this row; a chunk that a branch's
+        // last tile does not have counts for none
+        int a0, b0, a1, b1;
+        if (br != 1) {
+          const int j0 = (br == 0 ? 0 : sld_c0 * 64) + t * 128;
+          a0 = lo - j0; b0 = hi - j0; a1 = a0 - 64; b1 = b0 - 64;
+        } else if (OWN) {
+          const int blk = t < sel_cnt[rg] ? sel_list[rg * T5_MAX_SEL + t] : -1;
+          a0 = a1 = 0;
+          b0 = b1 = blk < 0 ? -1 : hi - blk * 64;
+        } else {
+          const int c1 = min(2 * t + 1, nchunks[1] - 1);
+          a0 = a1 = 0;
+          b0 = ((sel_mask[2 * t] >> rg) & 1) ? hi - sel_list[2 * t] * 64 : -1;
+          b1 = (c1 == 2 * t + 1 && ((sel_mask[c1] >> rg) & 1)) ? hi - sel_list[c1] * 64 : -1;
         }
         ok = __all_sync(0xffffffffu, mbar_wait(bar(B_SFULL + X), it & 1, &abort_flag));
         if (!ok) { fail_id = B_SFULL + X + 1; break; }
         tc_fence_after();
-        // the whole S row of the tile: 64*nch columns, one wait
+        // the whole S row of the tile in one round trip (columns of a missing second chunk hold what was there before: masked)
         uint32_t sv[4][32];
         tmem_ld32(tS + half * 64, sv[0]);
         tmem_ld32(tS + half * 64 + 32, sv[1]);
-        if (tl.nch == 2) { tmem_ld32(tS + 64, sv[2]); tmem_ld32(tS + 96, sv[3]); }
+        if (!own) { tmem_ld32(tS + 64, sv[2]); tmem_ld32(tS + 96, sv[3]); }
         tc_wait_ld();
         if constexpr (EARLY) {                             // S is in registers: the MMA warp may overwrite it
           tc_fence_before();
           mbar_arrive(bar(B_SREAD + X));
         }
-        // valid column range of each chunk for this row; masked entries become -inf
-        bool masked = false;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int vlo = max(lo - tl.j0[c], 0);
-          const int vhi = (c < tl.nch && ((tl.mask[c] >> rg) & 1)) ? min(hi, tl.jlim[c] - 1) - tl.j0[c] : -1;
-          if (c < tl.nch && (vlo > 0 || vhi < 63)) {
-            masked = true;
-#pragma unroll
-            for (int g = 0; g < 2; ++g)
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (g * 32 + i < vlo || g * 32 + i > vhi) sv[2 * c + g][i] = 0xff800000u;   // -inf
+        // masked entries become -inf
+        const bool masked = __any_sync(0xffffffffu, a0 > 0 || b0 < 63 || a1 > 0 || b1 < 63);
+        if (__builtin_expect(masked, 0)) {
+          mask_group(sv[0], 0, a0, b0);
+          mask_group(sv[1], 32, a0, b0);
+          if (!own) {
+            mask_group(sv[2], 0, a1, b1);
+            mask_group(sv[3], 32, a1, b1);
           }
         }
-        const bool use_poly = p.poly != 0 && !__any_sync(0xffffffffu, masked);
-        float mx = row_max_raw(sv, tl.nch);
+        const bool poly = !OWN && p.poly != 0 && !masked;     // warp-uniform
+        float mx = own ? row_max_raw<2>(sv) : row_max_raw<4>(sv);
         mx *= p.scale_log2[br];                              // scale > 0 keeps the order
         // lazy rescale: only when some row of the warp outgrows its reference maximum by 2^8
         const bool grow = mx > m_used + 8.f;
-        if (__any_sync(0xffffffffu, grow)) {
+        if (__builtin_expect(__any_sync(0xffffffffu, grow), 0)) {
           const float m_new = fmaxf(m_used, mx);
           const float alpha = m_new == -INFINITY ? 1.f : ex2(m_used - m_new);
           if (t > tbeg(br)) {
@@ -829,40 +840,21 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
         }
         const float m_ref = m_used == -INFINITY ? 0.f : m_used;
         // P = exp2(S*scale - m_ref) as 16-bit (-inf -> 0)
-        if (use_poly) {
-          const f32x2 SL = mk2(sl2, sl2), NM = mk2(-m_ref, -m_ref);
-          f32x2 sa = mk2(0.f, 0.f), sb = mk2(0.f, 0.f);
+        const f32x2 SL = mk2(sl2, sl2), NM = mk2(-m_ref, -m_ref);
+        f32x2 sa = mk2(0.f, 0.f), sb = mk2(0.f, 0.f);
+        auto sweep = [&](auto use_poly) {
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
-            if (g < 2 * tl.nch) {
-              exp_group_mixed<T>(sv[g], SL, NM, sa, sb);
-              if constexpr (!EARLY) tmem_st16(tP + half * 32 + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
-            }
+            if (g >= 2 && own) break;
+            exp_group<T, decltype(use_poly)::value>(sv[g], SL, NM, sa, sb);
+            if constexpr (!EARLY) tmem_st16(tP + half * 32 + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
             if (!EARLY && g == 1) { tc_wait_st(); tc_fence_before(); mbar_arrive(bar(B_PHALF + X)); }
           }
-          float s0, s1;
-          un2(add2(sa, sb), s0, s1);
-          l += s0 + s1;
-        } else {
-          float psum0 = 0.f, psum1 = 0.f, psum2 = 0.f, psum3 = 0.f;
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            if (g < 2 * tl.nch) {
-#pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const float p0 = ex2(fmaf(__uint_as_float(sv[g][2 * i]), sl2, -m_ref));
-                const float p1 = ex2(fmaf(__uint_as_float(sv[g][2 * i + 1]), sl2, -m_ref));
-                if (i & 1) { psum2 += p0; psum3 += p1; } else { psum0 += p0; psum1 += p1; }
-                sv[g][i] = Elem<T>::pack(p0, p1);
-              }
-              if constexpr (!EARLY) tmem_st16(tP + half * 32 + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
-            }
-            if (!EARLY && g == 1) { tc_wait_st(); tc_fence_before(); mbar_arrive(bar(B_PHALF + X)); }
-          }
-          psum0 += psum2;
-          psum1 += psum3;
-          l += psum0 + psum1;
-        }
+        };
+        if (__builtin_expect(poly, 1)) sweep(std::true_type{}); else sweep(std::false_type{});
+        float s0, s1;
+        un2(add2(sa, sb), s0, s1);
+        l += s0 + s1;
         if constexpr (EARLY) {
           // P's columns are free once the previous PV has read them: waited for here, with the exponentials done and packed, so
           // that PV runs under this tile's sweep and not before it (D=64, 64 heads over 4, T=16384: -2 %)
@@ -873,7 +865,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
           }
 #pragma unroll
           for (int g = 0; g < 4; ++g)
-            if (g < 2 * tl.nch) tmem_st16(tP + half * 32 + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
+            if (g < 2 || !own) tmem_st16(tP + half * 32 + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
         }
         tc_wait_st();
         tc_fence_before();
@@ -1507,38 +1499,41 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __gri
         const float sl2 = p.scale_log2[br];
 #pragma unroll 1
         for (int t = 0; t < ntiles(im, br) && ok; ++t, ++it) {
-          const Tile tl = get_tile(im, lp, br, t);
+          // columns a0..b0 of the tile's first 64 keys and a1..b1 of its second 64 count for this row; a chunk that a branch's
+          // last tile does not have counts for none
+          int a0, b0, a1, b1;
+          if (br != 1) {
+            const int j0 = (br == 0 ? 0 : im.sld_c0 * 64) + t * 128;
+            a0 = lo - j0; b0 = hi - j0; a1 = a0 - 64; b1 = b0 - 64;
+          } else {
+            const int c1 = min(2 * t + 1, im.nchunks[1] - 1);
+            a0 = a1 = 0;
+            b0 = ((sel_mask[lp][2 * t] >> rg) & 1) ? hi - sel_list[lp][2 * t] * 64 : -1;
+            b1 = (c1 == 2 * t + 1 && ((sel_mask[lp][c1] >> rg) & 1)) ? hi - sel_list[lp][c1] * 64 : -1;
+          }
           ok = __all_sync(0xffffffffu, mbar_wait(bar(B_SFULL + X), it & 1, &abort_flag));
           if (!ok) { fail_id = B_SFULL + X + 1; break; }
           tc_fence_after();
           uint32_t sv[4][32];
-          tmem_ld32(tS, sv[0]);
-          tmem_ld32(tS + 32, sv[1]);
-          if (tl.nch == 2) { tmem_ld32(tS + 64, sv[2]); tmem_ld32(tS + 96, sv[3]); }
+          #pragma unroll
+          for (int g = 0; g < 4; ++g) tmem_ld32(tS + g * 32, sv[g]);
           tc_wait_ld();
           if constexpr (EARLY) {
             tc_fence_before();
             mbar_arrive(bar(B_SREAD + X));
           }
-          bool masked = false;
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const int vlo = max(lo - tl.j0[c], 0);
-            const int vhi = (c < tl.nch && ((tl.mask[c] >> rg) & 1)) ? min(hi, tl.jlim[c] - 1) - tl.j0[c] : -1;
-            if (c < tl.nch && (vlo > 0 || vhi < 63)) {
-              masked = true;
-#pragma unroll
-              for (int g = 0; g < 2; ++g)
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                  if (g * 32 + i < vlo || g * 32 + i > vhi) sv[2 * c + g][i] = 0xff800000u;
-            }
+          const bool masked = __any_sync(0xffffffffu, a0 > 0 || b0 < 63 || a1 > 0 || b1 < 63);
+          if (__builtin_expect(masked, 0)) {
+            mask_group(sv[0], 0, a0, b0);
+            mask_group(sv[1], 32, a0, b0);
+            mask_group(sv[2], 0, a1, b1);
+            mask_group(sv[3], 32, a1, b1);
           }
-          const bool use_poly = p.poly != 0 && !__any_sync(0xffffffffu, masked);
-          float mx = row_max_raw(sv, tl.nch);
+          const bool poly = p.poly != 0 && !masked;
+          float mx = row_max_raw<4>(sv);
           mx *= p.scale_log2[br];
           const bool grow = mx > m_used + 8.f;
-          if (__any_sync(0xffffffffu, grow)) {
+          if (__builtin_expect(__any_sync(0xffffffffu, grow), 0)) {
             const float m_new = fmaxf(m_used, mx);
             const float alpha = m_new == -INFINITY ? 1.f : ex2(m_used - m_new);
             if (t > 0) {
@@ -1559,38 +1554,19 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __gri
             m_used = m_new;
           }
           const float m_ref = m_used == -INFINITY ? 0.f : m_used;
-          if (use_poly) {
-            const f32x2 SL = mk2(sl2, sl2), NM = mk2(-m_ref, -m_ref);
-            f32x2 sa = mk2(0.f, 0.f), sb = mk2(0.f, 0.f);
+          const f32x2 SL = mk2(sl2, sl2), NM = mk2(-m_ref, -m_ref);
+          f32x2 sa = mk2(0.f, 0.f), sb = mk2(0.f, 0.f);
+          auto sweep = [&](auto use_poly) {
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-              if (g < 2 * tl.nch) {
-                exp_group_mixed<T>(sv[g], SL, NM, sa, sb);
-                if constexpr (!EARLY) tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
-              }
+              exp_group<T, decltype(use_poly)::value>(sv[g], SL, NM, sa, sb);
+              if constexpr (!EARLY) tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
             }
-            float s0, s1;
-            un2(add2(sa, sb), s0, s1);
-            l += s0 + s1;
-          } else {
-            float psum0 = 0.f, psum1 = 0.f, psum2 = 0.f, psum3 = 0.f;
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              if (g < 2 * tl.nch) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                  const float p0 = ex2(fmaf(__uint_as_float(sv[g][2 * i]), sl2, -m_ref));
-                  const float p1 = ex2(fmaf(__uint_as_float(sv[g][2 * i + 1]), sl2, -m_ref));
-                  if (i & 1) { psum2 += p0; psum3 += p1; } else { psum0 += p0; psum1 += p1; }
-                  sv[g][i] = Elem<T>::pack(p0, p1);
-                }
-                if constexpr (!EARLY) tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
-              }
-            }
-            psum0 += psum2;
-            psum1 += psum3;
-            l += psum0 + psum1;
-          }
+          };
+          if (__builtin_expect(poly, 1)) sweep(std::true_type{}); else sweep(std::false_type{});
+          float s0, s1;
+          un2(add2(sa, sb), s0, s1);
+          l += s0 + s1;
           if constexpr (EARLY) {
             // P's columns are free once the previous PV has read them: waited for here, with the exponentials done and packed, so
             // that PV runs under this tile's sweep and not before it (D=64, 64 heads over 4, T=16384: -2 %)
@@ -1601,7 +1577,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __gri
             }
 #pragma unroll
             for (int g = 0; g < 4; ++g)
-              if (g < 2 * tl.nch) tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
+              tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
           }
           tc_wait_st();
           tc_fence_before();
@@ -1978,7 +1954,6 @@ int attention_fwd_tc5(const nsa_fwd_args& a, cudaStream_t st) {
     NSA_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));         \
     fn<<<(unsigned)blocks, T5_THREADS, smem, st>>>(p);                                                     \
   }
-    p.poly = 0;                        // every exponential on ex2, as on the mma.sync kernel
     if (fmt == 1) NSA_TC5_LAUNCH_OWN(1) else NSA_TC5_LAUNCH_OWN(0)
 #undef NSA_TC5_LAUNCH_OWN
     return launch_status("attn_fwd_tc5 (own lists)");

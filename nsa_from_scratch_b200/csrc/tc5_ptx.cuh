@@ -56,6 +56,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
 // Bounded wait: spins, then backs off with nanosleep; gives up (returns false) after about a
 // second or as soon as another thread of the block has raised `*abort_flag`.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
   for (int i = 0; i < 4096; ++i)
     if (mbar_try_wait(bar, parity)) return true;
   for (int i = 0; i < (1 << 22); ++i) {
