@@ -20,10 +20,10 @@
 //               gate/l and add it into the output row (the row itself holds the running gated sum)
 // TMEM columns: S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [384,384+D).
 // The softmax loop is laid out for instruction fetch: its unmasked path is one straight line (a wait that is over, the
-// load, the maximum, the exponentials by one route for all 128 columns), and masks, rescales and the all-ex2 route
-// stand behind branches marked unlikely.  Masking chunk by chunk and choosing per 32 columns in line, with the tile's description rebuilt
+// load, the maximum, the exponentials of all 128 columns), and masks and rescales stand behind branches marked
+// unlikely.  Masking chunk by chunk and choosing per 32 columns in line, with the tile's description rebuilt
 // by a three-way branch, the same work had its warps out of instructions for a third of their time (three warps per scheduler hide
-// no fetch): 64 heads over 4, T=16384: D=128 1594 -> 1496 us, D=64 1434 -> 1214 us.
+// no fetch): 64 heads over 4, T=16384: D=128 1594 -> 1496 us, D=64 1434 -> 1216 us.
 // Tile X's chain QK -> softmax -> PV is serial; the tensor pipe stays busy because the other
 // tile's MMAs run in the gaps.  Every mbarrier wait is bounded; a wait that gives up raises a
 // block-wide abort flag, sets the device status word and the block still frees its TMEM.
@@ -32,7 +32,6 @@
 
 #include <cudaTypedefs.h>
 #include <stdlib.h>
-#include <type_traits>
 
 namespace nsa {
 
@@ -61,7 +60,6 @@ struct Tc5Params {
   int tma_out;     // persistent kernel: an item whose result is ONE branch writes it through shared memory and the TMA (rows_through_tma)
   int fin_tma;     // one-item kernel, D = 128: the item's last branch end writes the output rows through shared memory and two TMA boxes per warp
   int psum;        // one-item kernel, unsplit 16-bit launches: 32 KB of shared memory hold the first 64 columns of the rows' running gated sum
-  int poly;        // tiles without masked entries take 3 of every 8 exponentials on the FMA pipe (exp2_poly_pair)
 };
 
 struct Tile {
@@ -93,25 +91,17 @@ __device__ __forceinline__ void mask_group(uint32_t (&s)[32], int c0, int vlo, i
 }
 
 // P = exp2(S * sl2 - m_ref) for 32 columns of a row, packed to 16-bit pairs in s[0..15]; the row sums go to the packed
-// accumulators.  POLY (columns without masked entries): of every 8 pairs, 3 are evaluated by the polynomial on the FMA pipe
-// and 5 by ex2 on the special-function unit: alone, a warp's sweep of 128 columns is bound by that unit (1024 of 1190
-// clocks); mixed this way it measured 947 clocks, and 2040 instead of 2410 with two warps sharing a scheduler.
-template <typename T, bool POLY>
+// accumulators.  All on the special-function unit (1024 of a tile's 3000 clocks and warp).  A cubic on the FMA pipe for 3 of
+// every 8 pairs relieved that unit but costs issue slots and 1.5 times the instructions to fetch: 64 heads over 4, T=16384,
+// D=128 1496 us with it, 1451 without (2 of 8: 1472, 1 of 8: 1457).
+template <typename T>
 __device__ __forceinline__ void exp_group(uint32_t (&s)[32], f32x2 SL, f32x2 NM, f32x2& sa, f32x2& sb) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    const f32x2 x = fma2(mk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), SL, NM);
-    float p0, p1;
-    if (POLY && (i & 7) < 3) {
-      exp2_poly_pair(x, p0, p1);
-    } else {
-      float x0, x1;
-      un2(x, x0, x1);
-      p0 = ex2(x0);
-      p1 = ex2(x1);
-    }
-    const f32x2 pp = mk2(p0, p1);
-    if (i & 1) sb = add2(sb, pp); else sa = add2(sa, pp);
+    float x0, x1;
+    un2(fma2(mk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), SL, NM), x0, x1);
+    const float p0 = ex2(x0), p1 = ex2(x1);
+    if (i & 1) sb = add2(sb, mk2(p0, p1)); else sa = add2(sa, mk2(p0, p1));
     s[i] = Elem<T>::pack(p0, p1);
   }
 }
@@ -163,7 +153,7 @@ enum { B_QFULL = 0, B_KFULL = 1, B_KEMPTY = 3, B_VFULL = 5, B_VEMPTY = 7, B_SFUL
 //
 // OWN (D = 64, one block list per query head): the four row groups of an item share no list.  Merged and masked, 3 of 4
 // (row, key) pairs of the selected branch were computed for nothing, and multi-head attention ran on the mma.sync kernel
-// instead (T=16384, 16 heads of their own keys, D=64: 591 us; this way 350).  A step of the selected branch takes the next
+// instead (T=16384, 16 heads of their own keys, D=64: 591 us; this way 333).  A step of the selected branch takes the next
 // listed block of EACH group: a ring slot holds four 64-key chunks, MMA tile X multiplies its 128 rows with the two chunks of
 // its own two groups, a softmax thread reads only its group's 64 columns of S, and the other group's 64 columns of P are zero,
 // so one N = 64 P V over both chunks adds to every row what its own chunk gives.  The tensor pipe does each product twice
@@ -775,21 +765,25 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
 #pragma unroll 1
       for (int t = tbeg(br); t < tend(br) && ok; ++t, ++it) {
         // columns a0..b0 of the tile's first 64 keys and a1..b1 of its second 64 count for this row; a chunk that a branch's
-        // last tile does not have counts for none
+        // last tile does not have counts for none.  Looked up while the row is on its way where the wait for S is short (D = 64:
+        // 1216 -> 1193 us there), ahead of that wait otherwise (the other way round: 1496 -> 1515 us).
         int a0, b0, a1, b1;
-        if (br != 1) {
-          const int j0 = (br == 0 ? 0 : sld_c0 * 64) + t * 128;
-          a0 = lo - j0; b0 = hi - j0; a1 = a0 - 64; b1 = b0 - 64;
-        } else if (OWN) {
-          const int blk = t < sel_cnt[rg] ? sel_list[rg * T5_MAX_SEL + t] : -1;
-          a0 = a1 = 0;
-          b0 = b1 = blk < 0 ? -1 : hi - blk * 64;
-        } else {
-          const int c1 = min(2 * t + 1, nchunks[1] - 1);
-          a0 = a1 = 0;
-          b0 = ((sel_mask[2 * t] >> rg) & 1) ? hi - sel_list[2 * t] * 64 : -1;
-          b1 = (c1 == 2 * t + 1 && ((sel_mask[c1] >> rg) & 1)) ? hi - sel_list[c1] * 64 : -1;
-        }
+        auto visible = [&]() {
+          if (br != 1) {
+            const int j0 = (br == 0 ? 0 : sld_c0 * 64) + t * 128;
+            a0 = lo - j0; b0 = hi - j0; a1 = a0 - 64; b1 = b0 - 64;
+          } else if (OWN) {
+            const int blk = t < sel_cnt[rg] ? sel_list[rg * T5_MAX_SEL + t] : -1;
+            a0 = a1 = 0;
+            b0 = b1 = blk < 0 ? -1 : hi - blk * 64;
+          } else {
+            const int c1 = min(2 * t + 1, nchunks[1] - 1);
+            a0 = a1 = 0;
+            b0 = ((sel_mask[2 * t] >> rg) & 1) ? hi - sel_list[2 * t] * 64 : -1;
+            b1 = (c1 == 2 * t + 1 && ((sel_mask[c1] >> rg) & 1)) ? hi - sel_list[c1] * 64 : -1;
+          }
+        };
+        if constexpr (!EARLY) visible();
         ok = __all_sync(0xffffffffu, mbar_wait(bar(B_SFULL + X), it & 1, &abort_flag));
         if (!ok) { fail_id = B_SFULL + X + 1; break; }
         tc_fence_after();
@@ -798,6 +792,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
         tmem_ld32(tS + half * 64, sv[0]);
         tmem_ld32(tS + half * 64 + 32, sv[1]);
         if (!own) { tmem_ld32(tS + 64, sv[2]); tmem_ld32(tS + 96, sv[3]); }
+        if constexpr (EARLY) visible();
         tc_wait_ld();
         if constexpr (EARLY) {                             // S is in registers: the MMA warp may overwrite it
           tc_fence_before();
@@ -813,7 +808,6 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
             mask_group(sv[3], 32, a1, b1);
           }
         }
-        const bool poly = !OWN && p.poly != 0 && !masked;     // warp-uniform
         float mx = own ? row_max_raw<2>(sv) : row_max_raw<4>(sv);
         mx *= p.scale_log2[br];                              // scale > 0 keeps the order
         // lazy rescale: only when some row of the warp outgrows its reference maximum by 2^8
@@ -842,16 +836,13 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
         // P = exp2(S*scale - m_ref) as 16-bit (-inf -> 0)
         const f32x2 SL = mk2(sl2, sl2), NM = mk2(-m_ref, -m_ref);
         f32x2 sa = mk2(0.f, 0.f), sb = mk2(0.f, 0.f);
-        auto sweep = [&](auto use_poly) {
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            if (g >= 2 && own) break;
-            exp_group<T, decltype(use_poly)::value>(sv[g], SL, NM, sa, sb);
-            if constexpr (!EARLY) tmem_st16(tP + half * 32 + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
-            if (!EARLY && g == 1) { tc_wait_st(); tc_fence_before(); mbar_arrive(bar(B_PHALF + X)); }
-          }
-        };
-        if (__builtin_expect(poly, 1)) sweep(std::true_type{}); else sweep(std::false_type{});
+        for (int g = 0; g < 4; ++g) {
+          if (g >= 2 && own) break;
+          exp_group<T>(sv[g], SL, NM, sa, sb);
+          if constexpr (!EARLY) tmem_st16(tP + half * 32 + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
+          if (!EARLY && g == 1) { tc_wait_st(); tc_fence_before(); mbar_arrive(bar(B_PHALF + X)); }
+        }
         float s0, s1;
         un2(add2(sa, sb), s0, s1);
         l += s0 + s1;
@@ -1500,23 +1491,28 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __gri
 #pragma unroll 1
         for (int t = 0; t < ntiles(im, br) && ok; ++t, ++it) {
           // columns a0..b0 of the tile's first 64 keys and a1..b1 of its second 64 count for this row; a chunk that a branch's
-          // last tile does not have counts for none
+          // last tile does not have counts for none.  Looked up while the row is on its way where the wait for S is short (D = 64:
+          // 1216 -> 1193 us there), ahead of that wait otherwise (the other way round: 1496 -> 1515 us).
           int a0, b0, a1, b1;
-          if (br != 1) {
-            const int j0 = (br == 0 ? 0 : im.sld_c0 * 64) + t * 128;
-            a0 = lo - j0; b0 = hi - j0; a1 = a0 - 64; b1 = b0 - 64;
-          } else {
-            const int c1 = min(2 * t + 1, im.nchunks[1] - 1);
-            a0 = a1 = 0;
-            b0 = ((sel_mask[lp][2 * t] >> rg) & 1) ? hi - sel_list[lp][2 * t] * 64 : -1;
-            b1 = (c1 == 2 * t + 1 && ((sel_mask[lp][c1] >> rg) & 1)) ? hi - sel_list[lp][c1] * 64 : -1;
-          }
+          auto visible = [&]() {
+            if (br != 1) {
+              const int j0 = (br == 0 ? 0 : im.sld_c0 * 64) + t * 128;
+              a0 = lo - j0; b0 = hi - j0; a1 = a0 - 64; b1 = b0 - 64;
+            } else {
+              const int c1 = min(2 * t + 1, im.nchunks[1] - 1);
+              a0 = a1 = 0;
+              b0 = ((sel_mask[lp][2 * t] >> rg) & 1) ? hi - sel_list[lp][2 * t] * 64 : -1;
+              b1 = (c1 == 2 * t + 1 && ((sel_mask[lp][c1] >> rg) & 1)) ? hi - sel_list[lp][c1] * 64 : -1;
+            }
+          };
+          if constexpr (!EARLY) visible();
           ok = __all_sync(0xffffffffu, mbar_wait(bar(B_SFULL + X), it & 1, &abort_flag));
           if (!ok) { fail_id = B_SFULL + X + 1; break; }
           tc_fence_after();
           uint32_t sv[4][32];
           #pragma unroll
           for (int g = 0; g < 4; ++g) tmem_ld32(tS + g * 32, sv[g]);
+          if constexpr (EARLY) visible();
           tc_wait_ld();
           if constexpr (EARLY) {
             tc_fence_before();
@@ -1529,7 +1525,6 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __gri
             mask_group(sv[2], 0, a1, b1);
             mask_group(sv[3], 32, a1, b1);
           }
-          const bool poly = p.poly != 0 && !masked;
           float mx = row_max_raw<4>(sv);
           mx *= p.scale_log2[br];
           const bool grow = mx > m_used + 8.f;
@@ -1556,14 +1551,11 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __gri
           const float m_ref = m_used == -INFINITY ? 0.f : m_used;
           const f32x2 SL = mk2(sl2, sl2), NM = mk2(-m_ref, -m_ref);
           f32x2 sa = mk2(0.f, 0.f), sb = mk2(0.f, 0.f);
-          auto sweep = [&](auto use_poly) {
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              exp_group<T, decltype(use_poly)::value>(sv[g], SL, NM, sa, sb);
-              if constexpr (!EARLY) tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
-            }
-          };
-          if (__builtin_expect(poly, 1)) sweep(std::true_type{}); else sweep(std::false_type{});
+          for (int g = 0; g < 4; ++g) {
+            exp_group<T>(sv[g], SL, NM, sa, sb);
+            if constexpr (!EARLY) tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
+          }
           float s0, s1;
           un2(add2(sa, sb), s0, s1);
           l += s0 + s1;
@@ -1828,11 +1820,6 @@ bool attention_fwd_tc5_supports(const nsa_fwd_args& a) {
 // 2.72, sliding 1.93 against 2.02); launches of several branches are 1-4 % slower on it than on the one-item kernel
 // (all three: 8.91-9.25 against 8.54-8.89 ms on the same box) and stay there, as do the split and fp8 launches.
 // NSA_TC5_PERSIST=0 / =1 in the environment forces the one-item / the persistent kernel for every unsplit 16-bit launch.
-// NSA_TC5_POLY=0 keeps every exponential on the special-function unit; default: 3 of 8 on the FMA pipe in unmasked tiles.
-static int tc5_poly_mode() {
-  static const int mode = [] { const char* e = getenv("NSA_TC5_POLY"); return !e ? 1 : (e[0] == '0' ? 0 : 1); }();
-  return mode;
-}
 static int tc5_persistent_mode() {
   static const int mode = [] { const char* e = getenv("NSA_TC5_PERSIST"); return !e ? -1 : (e[0] == '0' ? 0 : 1); }();
   return mode;
@@ -1856,7 +1843,6 @@ int attention_fwd_tc5(const nsa_fwd_args& a, cudaStream_t st) {
   }
   int rc;
   p.kv8 = in8 && a.kv_dtype == a.q_dtype;
-  p.poly = tc5_poly_mode();
   // NSA_TC5_KEEP_SUM=0: every branch end writes the whole running sum to the output row
   static const int psum_env = [] { const char* e = getenv("NSA_TC5_KEEP_SUM"); return !e ? 1 : (e[0] == '0' ? 0 : 1); }();
   p.psum = (psum_env && !in8 && !((a.nsplit > 1 || a.dyn_len != nullptr) && a.fused)) ? 1 : 0;
@@ -1916,8 +1902,8 @@ int attention_fwd_tc5(const nsa_fwd_args& a, cudaStream_t st) {
   const long long blocks = items * p.nsplit;
   NSA_REQUIRE(blocks > 0 && blocks < 2147483647LL, NSA_ERR_ARG, "attention forward: %lld work items do not fit a grid", blocks);
   // One block list per query head at D = 64: every row group walks its own list (OWN).  Against the mma.sync kernel, whole
-  // forwards of 16 heads with their own keys: T=512 52.9 against 50.6 us, 1024 73.1 / 74.3, 2048 75.6 / 94.6, 4096 129 / 164,
-  // 16384 438 / 629, 32768 890 / 1329; 16 heads over one, B=2, T=4001: 204 / 302 (four lists merged and masked: 383).
+  // forwards of 16 heads with their own keys: T=512 47 against 51 us, 1024 65 / 74, 2048 68 / 95, 4096 115 / 164,
+  // 16384 380 / 629; 16 heads over one, B=2, T=4001: 180 / 302 (four lists merged and masked: 361).
   // Launches that add to a 16-bit partial sum, and callers that name the engine, keep the merged lists: a branch added to
   // the rows afterwards and the same branches in one launch then give the same bits.
   const bool own = !in8 && !split && a.D == 64 && (a.branches & NSA_BRANCH_SELECTED) && a.Hi == a.H && a.engine == NSA_ENGINE_AUTO &&
