@@ -260,6 +260,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
     fence_barrier_init();
   }
   if (warp == 1) { tmem_alloc(smem_u32(&tmem_base_s), 512); tmem_relinquish(); }
+  if constexpr (OWN) grid_dep_wait();              // everything above runs while the launch before this one drains
   // scratch of the list builder: the first bytes of the (not yet used) Q tile area
   int* ent_blk = reinterpret_cast<int*>(smem);
   unsigned char* ent_p = smem + T5_MAX_ENT * sizeof(int);
@@ -1902,7 +1903,7 @@ int attention_fwd_tc5(const nsa_fwd_args& a, cudaStream_t st) {
   const long long blocks = items * p.nsplit;
   NSA_REQUIRE(blocks > 0 && blocks < 2147483647LL, NSA_ERR_ARG, "attention forward: %lld work items do not fit a grid", blocks);
   // One block list per query head at D = 64: every row group walks its own list (OWN).  Against the mma.sync kernel, whole
-  // forwards of 16 heads with their own keys: T=512 47 against 51 us, 1024 65 / 74, 2048 68 / 95, 4096 115 / 164,
+  // forwards of 16 heads with their own keys: T=512 45 against 51 us, 1024 62 / 74, 2048 68 / 95, 4096 111 / 164,
   // 16384 380 / 629; 16 heads over one, B=2, T=4001: 180 / 302 (four lists merged and masked: 361).
   // Launches that add to a 16-bit partial sum, and callers that name the engine, keep the merged lists: a branch added to
   // the rows afterwards and the same branches in one launch then give the same bits.
@@ -1934,15 +1935,15 @@ int attention_fwd_tc5(const nsa_fwd_args& a, cudaStream_t st) {
 #undef NSA_TC5_COMBINE
   }
   if (own) {
+    // through programmatic dependent launch: short sequences run here (16 heads x 512 46.5 -> 44.5 us, x 1024 63.0 -> 61.9)
 #define NSA_TC5_LAUNCH_OWN(FF)                                                                              \
   {                                                                                                         \
     auto fn = nsa_fwd_tc5_kernel<64, FF, false, false, true>;                                               \
     NSA_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));         \
-    fn<<<(unsigned)blocks, T5_THREADS, smem, st>>>(p);                                                     \
+    return launch_pdl("attn_fwd_tc5 (own lists)", fn, dim3((unsigned)blocks), T5_THREADS, smem, st, p);    \
   }
     if (fmt == 1) NSA_TC5_LAUNCH_OWN(1) else NSA_TC5_LAUNCH_OWN(0)
 #undef NSA_TC5_LAUNCH_OWN
-    return launch_status("attn_fwd_tc5 (own lists)");
   }
   const int n_br = ((a.branches >> 0) & 1) + ((a.branches >> 1) & 1) + ((a.branches >> 2) & 1);
   if (!in8 && (tc5_persistent_mode() == 1 || (tc5_persistent_mode() == -1 && n_br == 1))) {
