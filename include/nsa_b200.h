@@ -189,7 +189,8 @@ typedef struct nsa_fwd_args {
   /* Fused launches only.  accumulate != 0: `out` already holds a gated partial sum (an earlier fused launch with
    * other branches) and this launch adds its branches to it -- the three branches may thus be spread over several
    * launches, e.g. the compressed branch first when the selection is scored from its probabilities.  tcgen05 kernel
-   * only.  A fused launch of exactly ONE branch may also return that branch's lse (lse != NULL). */
+   * only.  A fused launch of exactly ONE branch may also return that branch's lse (lse != NULL); the compressed
+   * branch's is then formed as the block scores have always been formed with (within 2e-5 of the unfused launch's). */
   int32_t accumulate;
 } nsa_fwd_args;
 

@@ -106,6 +106,28 @@ __device__ __forceinline__ void exp_group(uint32_t (&s)[32], f32x2 SL, f32x2 NM,
   }
 }
 
+// The same for columns without masked entries with 3 of every 8 pairs on the FMA pipe.  The log-sum-exp that the block scores
+// are formed with keeps this arithmetic: it moves a row's sum by up to 1.6e-5, as much for one block as for the next, but
+// any other evaluation decides the scores that tie to fp32 rounding differently (two lists of 6144 at 64 heads over 4,
+// T=16384), and with them the blocks a caller's rows attend.
+template <typename T>
+__device__ __forceinline__ void exp_group_mixed(uint32_t (&s)[32], f32x2 SL, f32x2 NM, f32x2& sa, f32x2& sb) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const f32x2 x = fma2(mk2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), SL, NM);
+    float p0, p1;
+    if ((i & 7) < 3) {
+      exp2_poly_pair(x, p0, p1);
+    } else {
+      un2(x, p0, p1);
+      p0 = ex2(p0);
+      p1 = ex2(p1);
+    }
+    if (i & 1) sb = add2(sb, mk2(p0, p1)); else sa = add2(sa, mk2(p0, p1));
+    s[i] = Elem<T>::pack(p0, p1);
+  }
+}
+
 // End of a branch that alone makes up an item's result (single-branch launches), for one softmax warp: its 32 rows of
 // O (one thread per row in TMEM, D fp32 columns at tO) times the rows' coefficients, rounded to 16 bits, leave through a
 // 2 KB staging box (32 rows x 32 elements, 64-byte swizzle: 16-byte piece k of row r sits at piece k ^ ((r >> 1) & 3),
@@ -1022,7 +1044,8 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
 // 4*96 = 384: what the .inc calls take must have been released by the same block, or they block forever.
 enum { PB_LISTFULL = B_COUNT, PB_LISTEMPTY = B_COUNT + 2, PB_QFREE = B_COUNT + 4, PB_COUNT = B_COUNT + 5 };
 
-template <int D, int FMT>
+// MIXED: the launch whose log-sum-exp the block scores are formed with (exp_group_mixed in tiles without masked entries).
+template <int D, int FMT, bool MIXED>
 __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __grid_constant__ Tc5Params p, int n_items) {
   using T = typename std::conditional<FMT == 1, __nv_bfloat16, __half>::type;
   constexpr int DH = D / 64;
@@ -1520,6 +1543,8 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __gri
             mbar_arrive(bar(B_SREAD + X));
           }
           const bool masked = __any_sync(0xffffffffu, a0 > 0 || b0 < 63 || a1 > 0 || b1 < 63);
+          const bool two = !MIXED || 2 * t + 1 < im.nchunks[br];           // the tile's second chunk exists
+          const bool whole = MIXED && !__any_sync(0xffffffffu, a0 > 0 || b0 < 63 || (two && (a1 > 0 || b1 < 63)));
           if (__builtin_expect(masked, 0)) {
             mask_group(sv[0], 0, a0, b0);
             mask_group(sv[1], 32, a0, b0);
@@ -1552,11 +1577,23 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __gri
           const float m_ref = m_used == -INFINITY ? 0.f : m_used;
           const f32x2 SL = mk2(sl2, sl2), NM = mk2(-m_ref, -m_ref);
           f32x2 sa = mk2(0.f, 0.f), sb = mk2(0.f, 0.f);
+          auto exps = [&](auto mixed) {
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            exp_group<T>(sv[g], SL, NM, sa, sb);
-            if constexpr (!EARLY) tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
-          }
+            for (int g = 0; g < 4; ++g) {
+              if constexpr (decltype(mixed)::value) {
+                if (g < 2 || __builtin_expect(two, 1)) exp_group_mixed<T>(sv[g], SL, NM, sa, sb);
+                else {
+#pragma unroll
+                  for (int i = 0; i < 16; ++i) sv[g][i] = 0u;
+                }
+              } else exp_group<T>(sv[g], SL, NM, sa, sb);
+              if constexpr (!EARLY) tmem_st16(tP + g * 16, reinterpret_cast<const uint32_t (&)[16]>(sv[g]));
+            }
+          };
+          if constexpr (MIXED) {
+            if (__builtin_expect(whole, 1)) exps(std::true_type{});
+            else exps(std::false_type{});
+          } else exps(std::false_type{});
           float s0, s1;
           un2(add2(sa, sb), s0, s1);
           l += s0 + s1;
@@ -1946,7 +1983,9 @@ int attention_fwd_tc5(const nsa_fwd_args& a, cudaStream_t st) {
 #undef NSA_TC5_LAUNCH_OWN
   }
   const int n_br = ((a.branches >> 0) & 1) + ((a.branches >> 1) & 1) + ((a.branches >> 2) & 1);
-  if (!in8 && (tc5_persistent_mode() == 1 || (tc5_persistent_mode() == -1 && n_br == 1))) {
+  // A fused launch of the compressed branch alone that returns its log-sum-exp is what a scorer asks for
+  const bool scored = !in8 && a.fused && a.branches == NSA_BRANCH_COMPRESSED && a.lse != nullptr;
+  if (!in8 && (scored || tc5_persistent_mode() == 1 || (tc5_persistent_mode() == -1 && n_br == 1))) {
     // one thread block per SM walking the items (see nsa_fwd_tc5_persist_kernel)
     int dev = 0, sms = 0;
     NSA_CUDA_OK(cudaGetDevice(&dev));
@@ -1974,7 +2013,7 @@ int attention_fwd_tc5(const nsa_fwd_args& a, cudaStream_t st) {
     const size_t smem_p = (size_t)(2 + 2 + 2) * (a.D / 64) * 128 * 128 + (p.tma_out ? 8 * 2048 : 0) + 1024;
 #define NSA_TC5_PERSIST_LAUNCH(DD, FF)                                                                     \
   {                                                                                                         \
-    auto fn = nsa_fwd_tc5_persist_kernel<DD, FF>;                                                           \
+    auto fn = scored ? nsa_fwd_tc5_persist_kernel<DD, FF, true> : nsa_fwd_tc5_persist_kernel<DD, FF, false>; \
     NSA_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p));       \
     fn<<<grid, T5_THREADS, smem_p, st>>>(p, (int)blocks);                                                  \
   }

@@ -180,6 +180,27 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 d; asm("add.rn.f
 __device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { f32x2 d; asm("sub.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ float max3(float a, float b, float c) { float d; asm("max.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
 
+// 2^x for a pair of finite x on the FMA pipe: x is clamped to >= -125, split as n + f with n = round(x) (adding and
+// subtracting 1.5 * 2^23 leaves n in the low mantissa bits of t), 2^f on [-0.5, 0.5] by a cubic whose relative error is
+// 7.5e-5, and n added to the exponent field with integer arithmetic.  The result is never 0 (>= 2^-126): callers keep
+// masked (-inf) entries on ex2.  For the log-sum-exp behind the block scores only (exp_group_mixed).
+__device__ __forceinline__ void exp2_poly_pair(f32x2 x, float& p0, float& p1) {
+  const f32x2 MG = mk2(12582912.f, 12582912.f);
+  float x0, x1;
+  un2(x, x0, x1);
+  x = mk2(fmaxf(x0, -125.f), fmaxf(x1, -125.f));
+  const f32x2 t = add2(x, MG);
+  const f32x2 f = sub2(x, sub2(t, MG));
+  f32x2 q = fma2(mk2(0.0551716685295105f, 0.0551716685295105f), f, mk2(0.2426111251115799f, 0.2426111251115799f));
+  q = fma2(q, f, mk2(0.6932609677314758f, 0.6932609677314758f));
+  q = fma2(q, f, mk2(0.9999280571937561f, 0.9999280571937561f));
+  float q0, q1, t0, t1;
+  un2(q, q0, q1);
+  un2(t, t0, t1);
+  p0 = __uint_as_float(__float_as_uint(q0) + (__float_as_uint(t0) << 23));
+  p1 = __uint_as_float(__float_as_uint(q1) + (__float_as_uint(t1) << 23));
+}
+
 // ---------------------------------------------------------------- descriptors
 // Shared-memory matrix descriptor, 128-byte swizzle, sm_100 version field set.
 //   K-major operand  (rows x 64 elements per 128-byte row): sbo = bytes between 8-row groups (1024 when rows are dense)

@@ -41,8 +41,10 @@ def compressed_block_scores(Q: Tensor, K: Tensor, cfg) -> Tensor:
     scale = float(cfg.scale if cfg.scale is not None else 1.0 / (D ** 0.5))
     bc, stride, cmp_offset, nk, sel_offset = _geometry(cfg, Tq, Tk)
     Kc = ops.pool_mean(K.detach(), bc, stride)
-    # the compressed branch's log-sum-exp; its output is not needed, V stands in for the pooled values
-    _, lse = ops.attention_fwd(Q.detach(), K.detach(), K.detach(), branches=L.BRANCH_COMPRESSED, fused=False,
+    # the compressed branch's log-sum-exp; its output is not needed, V stands in for the pooled values.  A fused launch where
+    # there is one, as in forward_with_compressed_scorer: its log-sum-exp, and so the lists, are the same bit for bit
+    fused = ops.engine() != L.ENGINE_GENERIC and D in (64, 128) and scale > 0 and Kc.shape[2] > 0
+    _, lse = ops.attention_fwd(Q.detach(), K.detach(), K.detach(), branches=L.BRANCH_COMPRESSED, fused=fused, fused_lse=fused,
                                causal=bool(cfg.causal), scale=scale, Kc=Kc, Vc=Kc, cmp_block=bc, cmp_stride=stride,
                                cmp_offset=cmp_offset)
     return ops.cmp_block_scores(Q.detach(), Kc, lse, nk=nk, cmp_block=bc, cmp_stride=stride, cmp_offset=cmp_offset,
