@@ -14,7 +14,8 @@
 //
 // The gates enter through the log-sum-exp: the gradient of branch i's output is g_i dO, so with P' = g_i P = exp(S - lse +
 // ln g_i) both dV = P'^T dO and dS = P' (dP - d_i) hold with the ungated dO and d_i = dO . O_i.  Nothing of size
-// [rows, D] is written between the gated combine's gradient and these kernels.
+// [rows, D] is written between the gated combine's gradient and these kernels.  In fp16 a small gate would leave P' few
+// bits: there lse2 gives 2^14 P', and dS and the dV sums take the factor back (kGatedPExp).
 //
 // What bounds a step (128 x 64 pairs): 512 clocks of exp2 on the special-function unit, about 350 of issue slots, 384 to
 // 640 of MMAs; a step's own chain (MMA, TMEM load, exp2, TMEM store, MMA) is about 1700.  NBUF steps are therefore in flight,
@@ -50,8 +51,8 @@ struct BstParams {
   int B, H, Hkv, Hi, Tq, Tqp, Tk, Nc, nq, nk, top_k, G;
   int offset, cmp_offset, cmp_block, cmp_stride, sel_limit, window, causal;
   float scale, scale_log2;
-  const float* lse2;       // [3][B*H][Tqp]: log2-sum-exp minus log2 of the branch's gate
-  const float* dls;        // [3][B*H][Tqp]: (dO . O_branch) * scale
+  const float* lse2;       // [3][B*H][Tqp]: log2-sum-exp minus log2 of the branch's gate (fp16: minus kGatedPExp)
+  const float* dls;        // [3][B*H][Tqp]: (dO . O_branch) * scale (fp16: * kGatedPInv)
   const int32_t* idx;
   void* dQ;
   float *dK, *dV, *dKc, *dVc;   // [B*Hkv][Tk | Nc][D], added to
@@ -404,7 +405,7 @@ __global__ void __launch_bounds__(BST_THREADS, 1) nsa_bwd_stream_kernel(const __
     const int r = quarter * 32 + lane;                     // row of the 128-row tile == TMEM lane
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const uint32_t tS = tmem + lane_addr + grp * 128, tdP = tS + 64;
-    const float sc = p.scale, sl2 = p.scale_log2;
+    const float sc = FMT == 1 ? p.scale : p.scale * kGatedPInv, sl2 = p.scale_log2;
     const int g2 = r >> 6;
     bool ok = true;
 
@@ -567,12 +568,14 @@ __global__ void __launch_bounds__(BST_THREADS, 1) nsa_bwd_stream_kernel(const __
         } else {
           const int j = k0 + r, rows = br_k ? p.Tk : p.Nc;
           const bool isk = c >= D / 32;
+          const float fac = (FMT == 0 && !isk) ? kGatedPInv : 1.f;
           float* base = br_k ? (isk ? p.dK : p.dV) : (isk ? p.dKc : p.dVc);
           if (j < rows) {
             float* dst = base + ((size_t)owner * rows + j) * D + (c % (D / 32)) * 32;
 #pragma unroll
             for (int q = 0; q < 8; ++q)
-              red_add4(dst + q * 4, __uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]), __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]));
+              red_add4(dst + q * 4, __uint_as_float(v[4 * q]) * fac, __uint_as_float(v[4 * q + 1]) * fac, __uint_as_float(v[4 * q + 2]) * fac,
+                       __uint_as_float(v[4 * q + 3]) * fac);
           }
         }
       }
@@ -606,6 +609,8 @@ __global__ void __launch_bounds__(256) bwd_gates_kernel(const T* __restrict__ dO
                                                         float* __restrict__ lse2, float* __restrict__ dls, float* __restrict__ sel_lse,
                                                         float* __restrict__ sel_d, long long BH, int Tq, int Tqp, float scale) {
   constexpr int LPR = D / 8;
+  constexpr bool F16 = std::is_same<T, __half>::value;
+  constexpr float PX = F16 ? kGatedPExp : 0.f, PI = F16 ? kGatedPInv : 1.f;
   grid_dep_wait();
   const int sub = threadIdx.x % LPR;
   const long long rows_p = BH * Tqp, rows = BH * Tq;
@@ -669,8 +674,8 @@ __global__ void __launch_bounds__(256) bwd_gates_kernel(const T* __restrict__ dO
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const bool has = in && l[c] > -INFINITY;             // a row without a key in the branch takes no part: its P is masked
-      lse2[(size_t)c * rows_p + pr] = has ? (l[c] - lg[c]) * kLog2e : 0.f;
-      dls[(size_t)c * rows_p + pr] = has ? d[c] * scale : 0.f;
+      lse2[(size_t)c * rows_p + pr] = has ? (l[c] - lg[c]) * kLog2e - PX : 0.f;
+      dls[(size_t)c * rows_p + pr] = has ? d[c] * (scale * PI) : 0.f;
       if (in && dgates != nullptr) {
         if (gate_dtype == NSA_FP32) reinterpret_cast<float*>(dgates)[row * 3 + c] = dx[c];
         else if (gate_dtype == NSA_FP16) reinterpret_cast<__half*>(dgates)[row * 3 + c] = __float2half_rn(dx[c]);

@@ -50,6 +50,8 @@ struct Bw5Params {
   CUtensorMap tmQ, tmdO, tmK, tmV;
   nsa_bwd_args a;
   float scale_log2;
+  // P is formed as 2^p_exp P: dS takes scale * 2^-p_exp, the dV sums 2^-p_exp (0 and 1 outside the whole forward's backward)
+  float p_exp, ds_scale, dv_scale;
   int nkb;                 // key blocks
   int G;                   // query heads per KV head
   int shared;              // one block list per KV head (1) or per query head (0)
@@ -373,7 +375,7 @@ __global__ void __launch_bounds__(BW5_THREADS, 1) nsa_bwd_tc5_kernel(const __gri
     const int g2 = r >> 6;
     const uint32_t tS = tmem + lane_addr + grp * 128 + hf * 32, tdP = tS + 64;
     unsigned char* prow = pb_ptr + grp * PB_BYTES + r * 128;           // this row of P (key-major) / dS (query-major)
-    const float sc = a.scale;
+    const float sc = p.ds_scale;
 
     // What a query row needs: its log-sum-exp (log2 units), delta*scale, and the last key position it may see.
     // Query-major: the row is fixed.  Key-major: the rows change every step and come through two dependent loads
@@ -400,7 +402,7 @@ __global__ void __launch_bounds__(BW5_THREADS, 1) nsa_bwd_tc5_kernel(const __gri
     auto adopt = [&](const RowRaw& rr) {
       lse2 = 0.f; dls = 0.f; hi = -1;
       if (rr.ok && rr.l > -INFINITY) {
-        lse2 = rr.l * kLog2e;
+        lse2 = rr.l * kLog2e - p.p_exp;
         dls = rr.d * sc;
         hi = a.causal ? min(rr.qi + a.offset, a.sel_key_limit - 1) : a.sel_key_limit - 1;
       }
@@ -515,13 +517,14 @@ __global__ void __launch_bounds__(BW5_THREADS, 1) nsa_bwd_tc5_kernel(const __gri
         if (direct) dst = (which ? a.dK_f : a.dV_f) + ((size_t)kv_slab * a.Tk + key) * D + part * HC;
         else dst = p.partials + ((((size_t)owner * p.capP + slot) * 2 + which) * 64 + kr) * D + part * HC;
         const bool wr = !direct || key < a.Tk;
+        const float fac = which ? 1.f : p.dv_scale;
         uint32_t v[HC];
         load_part(tmem + lane_addr + 256 + which * D + part * HC, v);
         if (wr) {
 #pragma unroll
           for (int q4 = 0; q4 < HC / 4; ++q4) {
-            float4 o = make_float4(__uint_as_float(v[4 * q4]), __uint_as_float(v[4 * q4 + 1]), __uint_as_float(v[4 * q4 + 2]),
-                                   __uint_as_float(v[4 * q4 + 3]));
+            float4 o = make_float4(__uint_as_float(v[4 * q4]) * fac, __uint_as_float(v[4 * q4 + 1]) * fac, __uint_as_float(v[4 * q4 + 2]) * fac,
+                                   __uint_as_float(v[4 * q4 + 3]) * fac);
             float4* dp4 = reinterpret_cast<float4*>(dst) + q4;
             if (direct) { const float4 old = *dp4; o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w; }
             *dp4 = o;
@@ -807,7 +810,8 @@ static Bw5Plan bw5_plan(const nsa_bwd_args& a) {
 
 long long attention_bwd_tc5_scratch_bytes(const nsa_bwd_args& a) { return (long long)bw5_plan(a).total; }
 
-// keys_only: dK and dV alone (the whole forward's backward forms dQ in its own pass over all branches)
+// keys_only: dK and dV alone (the whole forward's backward forms dQ in its own pass over all branches).  Its log-sum-exps carry
+// the gates, so P is gate * P; fp16 storage scales it as the streaming passes do.
 int attention_bwd_tc5(const nsa_bwd_args& a, void* scratch, long long scratch_bytes, bool keys_only, cudaStream_t st) {
   const Bw5Plan pl = bw5_plan(a);
   NSA_REQUIRE(scratch != nullptr && scratch_bytes >= (long long)pl.total, NSA_ERR_ARG,
@@ -826,6 +830,10 @@ int attention_bwd_tc5(const nsa_bwd_args& a, void* scratch, long long scratch_by
   Bw5Params p;
   p.a = a;
   p.scale_log2 = a.scale * kLog2e;
+  const bool up = keys_only && a.dtype == NSA_FP16;
+  p.p_exp = up ? kGatedPExp : 0.f;
+  p.dv_scale = up ? kGatedPInv : 1.f;
+  p.ds_scale = a.scale * p.dv_scale;
   p.nkb = pl.nkb; p.G = pl.G; p.shared = pl.shared;
   p.items = items; p.n_items = n_items; p.capW = pl.capW; p.rg_list = rg_list; p.cap_rg = pl.cap_rg;
   p.partials = partials; p.capP = pl.capP;

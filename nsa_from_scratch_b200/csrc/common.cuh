@@ -67,6 +67,11 @@ struct PoolJob {
   unsigned block0;     // filled in by the launcher
 };
 
+// Backward of the whole forward, fp16 storage: gate * P, which has no gate-independent size, is held as 2^14 times itself.  It is
+// at most 1, so nothing overflows, and values down to 4e-9 keep all 11 bits (unscaled: 6e-5, which gate logits of -6
+// over a few thousand keys fall below, and no scaling of the loss can reach).  bf16 has the exponents of fp32.
+constexpr float kGatedPExp = 14.f, kGatedPInv = 1.f / 16384.f;
+
 // ---------------------------------------------------------------- dtype traits
 template <typename T> struct Elem;
 template <> struct Elem<__nv_bfloat16> {

@@ -60,3 +60,40 @@ def test_gradients_vs_oracle(nsa, case):
         assert err <= 2e-2 * max(1.0, mag), (name, err, mag)
     again = torch.autograd.grad(nsa.nsa_forward(*dev[:3], cfg, gate_logits=None if gates is None else dev[3]), dev, dO.cuda())
     assert torch.equal(again[0], got[0])                 # dQ is formed in a fixed order
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("logit", [0.0, -4.0, -8.0])
+def test_fp16_small_gates_keep_their_bits(nsa, D, logit):
+    """gate * P in fp16: at 4096 keys and logits of -8 it lies far below the smallest normal number, and scaling dO does not
+    change it.  Relative error of the gradients against 64 bits: an operand rounded to 11 bits is off by 2^-12 / sqrt(3) on
+    average, 1.4e-4, two to four of them come together; bound 5e-4."""
+    T, H, W = 4096, 2, 256
+    Q, K, V, g = make_qkv(17, 1, H, 1, T, T, D, dtype=torch.float16)
+    gates = (logit + 0.3 * torch.randn(1, H, T, 3, generator=g)).cuda()
+    dO = (torch.randn(1, H, T, D, generator=g).half() * (1.0 if logit == 0.0 else 1024.0)).cuda()
+    cfg = nsa.NSAConfig(block_size_c=32, stride_c=16, top_k=8, window_size=W, select_per_group=True)
+    leaves = [t.cuda().requires_grad_(True) for t in (Q, K, V)]
+    idx = nsa._resolve_block_indices(*leaves[:2], block_size_m=64, block_size_n=64, top_k=8, causal=True, scale=D ** -0.5, shared_per_group=True)
+    got = torch.autograd.grad(nsa.nsa_forward(*leaves, cfg, gate_logits=gates, block_indices=idx), leaves, dO)
+    q, k, v = (t.detach().double().requires_grad_(True) for t in leaves)
+    pos, n = torch.arange(T, device="cuda"), (T - 32) // 16 + 1
+    at = pos[None] - 16 * torch.arange(n, device="cuda")[:, None]
+    pool = ((at >= 0) & (at < 32)).double() / 32
+    def pooled(x):                                        # the kernels read pooled rows rounded to 16 bits
+        y = pool @ x[0, 0]
+        return y + (y.detach().half().double() - y.detach())
+    past = pos[None] <= pos[:, None]
+    listed = torch.zeros(T // 64, T // 64, dtype=torch.bool, device="cuda").scatter_(1, idx[0, 0].long(), True)
+    masks = (16 * torch.arange(n, device="cuda")[None] + 31 <= pos[:, None], past & listed.repeat_interleave(64, 0).repeat_interleave(64, 1),
+             past & (pos[None] > pos[:, None] - W))
+    keys = ((pooled(k), pooled(v)), (k[0, 0], v[0, 0]), (k[0, 0], v[0, 0]))
+    total = 0.0
+    for h in range(H):
+        for c in range(3):
+            s = (q[0, h] @ keys[c][0].T * D ** -0.5).masked_fill(~masks[c], -1e30)
+            p = torch.softmax(s, -1).masked_fill(~masks[c], 0.0)
+            total = total + (torch.sigmoid(gates[0, h, :, c:c + 1].double()) * (p @ keys[c][1]) * dO[0, h].double()).sum()
+    for name, a, r in zip(("dQ", "dK", "dV"), got, torch.autograd.grad(total, (q, k, v))):
+        err = float((a.double() - r).norm() / r.norm())
+        assert err <= 5e-4, (name, err)
