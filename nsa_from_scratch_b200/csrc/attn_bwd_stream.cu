@@ -814,7 +814,7 @@ static int bst_launch(const nsa_forward_args& f, const BstPlan& pl, BstParams& p
   p.kt_cmp = (pl.Nc + 127) / 128;
   p.kt_sld = (f.Tk + 127) / 128;
   const long long most_cmp = (long long)pl.nq * p.G;                     // steps of a pooled key tile that every query sees
-  const long long most_sld = (long long)((128 + (f.causal ? 1 : 2) * (long long)f.window) / 64 + 2) * p.G;
+  const long long most_sld = (long long)((128 + (f.causal ? 1 : 2) * (long long)p.window) / 64 + 2) * p.G;
   const long long total = NL * (p.kt_cmp * most_cmp / 2 + p.kt_sld * (most_sld < most_cmp ? most_sld : most_cmp));
   long long L = total / ((long long)sms * 8);
   p.L = (int)(L < 32 ? 32 : (L > 256 ? 256 : L));
@@ -850,7 +850,10 @@ int backward_stream(const nsa_forward_args& f, const void* dO, const void* branc
   p.top_k = pl.k_sel; p.G = f.H / f.Hkv;
   p.offset = f.Tk - f.Tq;
   p.cmp_offset = (f.cmp_stride == f.cmp_block ? pl.Nc * f.cmp_block : f.Tk) - f.Tq;
-  p.cmp_block = f.cmp_block; p.cmp_stride = f.cmp_stride; p.sel_limit = pl.nk * 64; p.window = f.window; p.causal = f.causal;
+  p.cmp_block = f.cmp_block; p.cmp_stride = f.cmp_stride; p.sel_limit = pl.nk * 64; p.causal = f.causal;
+  // a window beyond the sequence ("no window", up to INT_MAX) hides no key: cut to it, so that positions plus window stay in range
+  const int reach = f.Tq > f.Tk ? f.Tq : f.Tk;
+  p.window = f.window < reach ? f.window : reach;
   p.scale = f.scale; p.scale_log2 = f.scale * kLog2e;
   p.lse2 = reinterpret_cast<float*>(ws + pl.o_lse2);
   p.dls = reinterpret_cast<float*>(ws + pl.o_dls);

@@ -97,3 +97,19 @@ def test_fp16_small_gates_keep_their_bits(nsa, D, logit):
     for name, a, r in zip(("dQ", "dK", "dV"), got, torch.autograd.grad(total, (q, k, v))):
         err = float((a.double() - r).norm() / r.norm())
         assert err <= 5e-4, (name, err)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_window_beyond_the_sequence(nsa, D):
+    """2**31 - 1 for "no window": the gradients of a window that just covers the sequence.  dQ repeats bit for bit; dK and dV are
+    fp32 sums in another order, rounded to 8 bits: 1e-3 of the norm (a bf16 ulp of 4e-3 here and there)."""
+    Q, K, V, g = make_qkv(23, 1, 4, 2, 300, 333, D)
+    dO = torch.randn(1, 4, 300, D, generator=g).bfloat16().cuda()
+    grads = []
+    for window in (333, 2**31 - 1):
+        cfg = nsa.NSAConfig(block_size_c=32, stride_c=16, top_k=2, window_size=window, select_per_group=True)
+        leaves = [t.cuda().requires_grad_(True) for t in (Q, K, V)]
+        grads.append(torch.autograd.grad(nsa.nsa_forward(*leaves, cfg), leaves, dO))
+    assert torch.equal(grads[0][0], grads[1][0])
+    for a, b in zip(*(x[1:] for x in grads)):
+        assert float((a.float() - b.float()).norm() / a.float().norm()) <= 1e-3
