@@ -177,9 +177,10 @@ enum { B_QFULL = 0, B_KFULL = 1, B_KEMPTY = 3, B_VFULL = 5, B_VEMPTY = 7, B_SFUL
 // (row, key) pairs of the selected branch were computed for nothing, and multi-head attention ran on the mma.sync kernel
 // instead (T=16384, 16 heads of their own keys, D=64: 591 us; this way 333).  A step of the selected branch takes the next
 // listed block of EACH group: a ring slot holds four 64-key chunks, MMA tile X multiplies its 128 rows with the two chunks of
-// its own two groups, a softmax thread reads only its group's 64 columns of S, and the other group's 64 columns of P are zero,
-// so one N = 64 P V over both chunks adds to every row what its own chunk gives.  The tensor pipe does each product twice
-// over, which costs nothing here: it is busy 20 % of the time, the softmax warps' serial sweep is what a step takes.
+// its own two groups, a softmax thread reads only its group's 64 columns of S, and the P V of a chunk leaves the other group's
+// lanes of O as they are, so a row takes nothing from a block that it does not list -- not even 0 times an infinity.  The tensor
+// pipe does each product twice over, which costs nothing here: it is busy 20 % of the time, the softmax warps' serial sweep is
+// what a step takes.
 // The running gated sum is held in fp32 in shared memory: D = 64 leaves the room, and the result is rounded once.
 template <int D, int FMT, bool IN8, bool SPLIT, bool OWN = false>
 __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_constant__ Tc5Params p) {
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
           }
           if constexpr (OWN) {
             if (br == 1) {
-              // the next listed block of each row group; a group whose list has ended gets block 0, masked out by its rows
+              // the next listed block of each row group; a group whose list has ended gets block 0, which no row takes
               int j0[4];
 #pragma unroll
               for (int g = 0; g < 4; ++g) j0[g] = t < sel_cnt[g] ? sel_list[g * T5_MAX_SEL + t] * 64 : 0;
@@ -545,6 +546,11 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
       const uint32_t tSx[2] = {tmem, tmem + 128}, tOx[2] = {tmem + 256, tmem + 384};
       const uint32_t tPx[2] = {EARLY ? tmem + 320 : tmem, EARLY ? tmem + 448 : tmem + 128};
 
+      int own_cnt[4] = {0, 0, 0, 0};                       // own lists: entries of each row group
+      if (OWN && (a.branches & NSA_BRANCH_SELECTED)) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) own_cnt[g] = sel_cnt[g];
+      }
       // position of the tile whose QK is issued next / whose PV is issued next (tile tbeg(br) + t of the branch)
       int q_br = 0, q_t = 0, p_br = 0, p_t = 0;
       auto skip_empty = [&](int& br, int& t) { while (br < 3 && t >= nt_of[br]) { ++br; t = 0; } };
@@ -580,6 +586,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
       for (int it = 0; it < total_tiles && ok; ++it) {
         const int nch = min(2, nchunks[p_br] - 2 * (tbeg(p_br) + p_t));
         const bool fresh = p_t == 0;                       // first tile of a branch starts a new O
+        const bool own_pv = OWN && p_br == 1;
         const int s = it & 1;
         ok = __all_sync(0xffffffffu, mbar_wait(bar(B_VFULL + s), (it >> 1) & 1, &abort_flag));
         if (!ok) { fail_id = B_VFULL + s + 1; break; }
@@ -597,7 +604,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
 #pragma unroll
         for (int X = 0; X < 2; ++X) {
           if (!ok) break;
-          const uint64_t dVs = dV[s] + ((OWN && p_br == 1) ? X * (KVTILE >> 4) : 0);
+          const uint64_t dVs = dV[s] + (own_pv ? X * (KVTILE >> 4) : 0);
           if constexpr (!EARLY) {
             // first 64 keys of P V as soon as that half of P is written
             ok = __all_sync(0xffffffffu, mbar_wait_spin(bar(B_PHALF + X), it & 1, &abort_flag));
@@ -615,15 +622,26 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
           if (!ok) { fail_id = B_PFULL + X + 1; break; }
           tc_fence_after();
           if (leader) {
-            if constexpr (EARLY) {
-              if (fresh) mma_ts(tOx[X], tPx[X], dVs, IDESC_PV, 0u);
-              else mma_ts(tOx[X], tPx[X], dVs, IDESC_PV, 1u);
+            if (own_pv) {
+              // a chunk at a time, into its own group's 64 lanes; a group whose list has ended keeps its O
 #pragma unroll
-              for (int kk = 1; kk < 4; ++kk) mma_ts(tOx[X], tPx[X] + kk * 8, dVs + kk * 128, IDESC_PV, 1u);
-            }
-            if (nch == 2) {
+              for (int h = 0; h < 2; ++h)
+                if (p_t < own_cnt[2 * X + h]) {
 #pragma unroll
-              for (int kk = 4; kk < 8; ++kk) mma_ts(tOx[X], tPx[X] + kk * 8, dVs + kk * 128, IDESC_PV, 1u);
+                  for (int kk = 4 * h; kk < 4 * h + 4; ++kk)
+                    mma_ts_half(tOx[X], tPx[X] + kk * 8, dVs + kk * 128, IDESC_PV, fresh && kk == 4 * h ? 0u : 1u, h);
+                }
+            } else {
+              if constexpr (EARLY) {
+                if (fresh) mma_ts(tOx[X], tPx[X], dVs, IDESC_PV, 0u);
+                else mma_ts(tOx[X], tPx[X], dVs, IDESC_PV, 1u);
+#pragma unroll
+                for (int kk = 1; kk < 4; ++kk) mma_ts(tOx[X], tPx[X] + kk * 8, dVs + kk * 128, IDESC_PV, 1u);
+              }
+              if (nch == 2) {
+#pragma unroll
+                for (int kk = 4; kk < 8; ++kk) mma_ts(tOx[X], tPx[X] + kk * 8, dVs + kk * 128, IDESC_PV, 1u);
+              }
             }
             tc_commit(bar(B_PVDONE + X));
             if (X == 1) tc_commit(bar(B_VEMPTY + s));
@@ -775,15 +793,6 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
       float m_used = -INFINITY, l = 0.f;
       const bool own = OWN && br == 1;
       const int half = own ? quarter >> 1 : 0;             // own lists: this row's 64 columns of S and P
-      if constexpr (OWN) {
-        if (own) {                                         // the other group's columns of P stay zero for the whole branch
-          uint32_t z[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) z[i] = 0u;
-          tmem_st16(tP + (half ^ 1) * 32, z);
-          tmem_st16(tP + (half ^ 1) * 32 + 16, z);
-        }
-      }
       const float sl2 = p.scale_log2[br];
 #pragma unroll 1
       for (int t = tbeg(br); t < tend(br) && ok; ++t, ++it) {
@@ -940,7 +949,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
                 for (int e = 0; e < 8; ++e) acc[e] = 0.f;
               }
 #pragma unroll
-              for (int e = 0; e < 8; ++e) acc[e] = fmaf(__uint_as_float(v[8 * c + e]), coef, acc[e]);
+              for (int e = 0; e < 8; ++e) acc[e] = has ? fmaf(__uint_as_float(v[8 * c + e]), coef, acc[e]) : acc[e];   // no key: O was not written
               if (br != last_br) {
                 *q0 = make_float4(acc[0], acc[1], acc[2], acc[3]);
                 *q1 = make_float4(acc[4], acc[5], acc[6], acc[7]);

@@ -46,3 +46,25 @@ def test_forward_and_selected_branch(nsa, H, Hkv, Tq, Tk, k, window, dtype):
     out = nsa.nsa_forward(q, kk, v, cfg, gate_logits=gates.cuda(), block_indices=i)
     ref = O.nsa_forward(Q, K, V, block_size_c=32, stride_c=16, top_k=k, window_size=window, gate_logits=gates, block_indices=idx)
     assert max_abs(out, ref) <= 2e-2, max_abs(out, ref)
+
+
+@pytest.mark.parametrize("H,Hkv", [(3, 3), (4, 2), (8, 2)])
+@pytest.mark.parametrize("block", [0, 5])                  # 0 also stands in for the entries of a list that has ended
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_rows_take_nothing_from_blocks_they_do_not_list(nsa, H, Hkv, block, bad):
+    T = 1024
+    Q, K, V, _ = make_qkv(8, 1, H, Hkv, T, T, 64)
+    g = torch.Generator().manual_seed(4)
+    idx = torch.randint(0, 15, (1, H, 16, 4), generator=g, dtype=torch.int32)
+    idx += (idx >= block).int()                             # every block but `block`
+    idx[torch.rand(idx.shape, generator=g) < 0.3] = -1
+    idx[:, :, 11] = -1
+    idx[:, 1, 9, 2] = block                                 # one list names it
+    poisoned = V.clone()
+    poisoned[:, :, block * 64 + 7] = bad
+    out, lse = (x.cpu() for x in nsa.selected_attention(Q.cuda(), K.cuda(), V.cuda(), top_k=4, block_indices=idx.cuda(), causal=False))
+    got, glse = (x.cpu() for x in nsa.selected_attention(Q.cuda(), K.cuda(), poisoned.cuda(), top_k=4, block_indices=idx.cuda(), causal=False))
+    rows = torch.ones(1, H, T, dtype=torch.bool)
+    rows[:, 1, 9 * 64:10 * 64] = False
+    assert torch.equal(glse, lse) and torch.equal(got[rows], out[rows])
+    assert not torch.isfinite(got[~rows]).any()
