@@ -285,19 +285,32 @@ def attention_fwd(
     return out, lse
 
 
-# nsa_forward_args of the problems seen so far, pointers left out: (bytes of the struct, workspace bytes of the forward,
-# of the backward (0: not taken), shape of the block lists, pooled tokens)
+# nsa_forward_args of the problems seen so far, pointers and scales left out: (bytes of the struct, workspace bytes of the
+# forward, of the backward (0: not taken), shape of the block lists, pooled tokens).  The scales (a caller may quantise anew for
+# every call, or keep one in a tensor that it updates) decide by their signs alone which kernels run.
 _forward_plans: dict = {}
 
 
 def forward_plan(q_shape, k_shape, dtype, *, causal: bool, scale: float, cmp_block: int, cmp_stride: int, bm: int, bn: int, window: int,
                  top_k: int, force_first: int, force_local: int, per_group: bool, idx_shape, gate_dtype, gate_act: int, q_scale: float,
                  k_scale: float, v_scale: float, engine: int, token_major: bool):
-    key = (q_shape, k_shape, dtype, causal, scale, cmp_block, cmp_stride, bm, bn, window, top_k, force_first, force_local, per_group,
-           idx_shape, gate_dtype, gate_act, q_scale, k_scale, v_scale, engine, token_major)
+    """(nsa_forward_args without pointers, ...): a fresh struct with this call's scales, then what _forward_plans keeps."""
+    scales = float(scale), float(q_scale), float(k_scale), float(v_scale)
+    window = int(window)
+    key = (q_shape, k_shape, dtype, causal, cmp_block, cmp_stride, bm, bn, window, top_k, force_first, force_local, per_group, idx_shape,
+           gate_dtype, gate_act, engine, token_major, *[x > 2.0**-150 for x in scales])      # positive as a 32-bit float
     plan = _forward_plans.get(key)
-    if plan is not None:
-        return plan
+    if plan is None:
+        plan = _plan_forward(key, scales, q_shape, k_shape, dtype, causal=causal, cmp_block=cmp_block, cmp_stride=cmp_stride, bm=bm, bn=bn,
+                             window=window, top_k=top_k, force_first=force_first, force_local=force_local, per_group=per_group,
+                             idx_shape=idx_shape, gate_dtype=gate_dtype, gate_act=gate_act, engine=engine, token_major=token_major)
+    a = L.ForwardArgs.from_buffer_copy(plan[0])
+    a.scale, a.q_scale, a.k_scale, a.v_scale = scales
+    return (a, *plan[1:])
+
+
+def _plan_forward(key, scales, q_shape, k_shape, dtype, *, causal, cmp_block, cmp_stride, bm, bn, window, top_k, force_first, force_local,
+                  per_group, idx_shape, gate_dtype, gate_act, engine, token_major):
     B, H, Tq, D = q_shape
     Hkv, Tk = k_shape[1], k_shape[2]
     if k_shape != (B, Hkv, Tk, D):
@@ -314,11 +327,11 @@ def forward_plan(q_shape, k_shape, dtype, *, causal: bool, scale: float, cmp_blo
         a.has_idx, a.Hi, a.top_k = 1, idx_shape[1], idx_shape[3]
     else:
         idx_shape = (B, Hkv if per_group else H, nq, min(int(top_k), nk))
-    a.cmp_block, a.cmp_stride, a.bm, a.bn, a.window, a.causal = cmp_block, cmp_stride, bm, bn, int(window), int(causal)
+    a.cmp_block, a.cmp_stride, a.bm, a.bn, a.window, a.causal = cmp_block, cmp_stride, bm, bn, window, int(causal)
     a.gate_act, a.q_dtype, a.engine = gate_act, L.dtype_code(dtype), engine
     a.gate_dtype = 0 if gate_dtype is None else L.dtype_code(gate_dtype)
     a.io_layout = (L.IO_OUT_BTHD | L.IO_GATES_BTHD) if token_major else 0
-    a.scale, a.q_scale, a.k_scale, a.v_scale = float(scale), float(q_scale), float(k_scale), float(v_scale)
+    a.scale, a.q_scale, a.k_scale, a.v_scale = scales
     lib = L.load()
     need = int(lib.nsa_forward_ws_bytes(C.byref(a)))
     if need < 0:
@@ -356,7 +369,7 @@ def forward(Q: Tensor, K: Tensor, V: Tensor, *, idx: Optional[Tensor] = None, ga
     plan = forward_plan(Q.shape, K.shape, dtype, idx_shape=None if idx is None else idx.shape, gate_dtype=None if gates is None else gates.dtype,
                         q_scale=q_scale, k_scale=k_scale, v_scale=v_scale, engine=_ENGINE if engine is None else engine,
                         token_major=token_major, **geometry)
-    a = L.ForwardArgs.from_buffer_copy(plan[0])
+    a = plan[0]
     B, H, Tq, D = Q.shape
     dev = Q.device
     out = torch.empty((B, Tq, H, D) if token_major else (B, H, Tq, D), device=dev, dtype=torch.bfloat16 if dtype in _8 else dtype)
