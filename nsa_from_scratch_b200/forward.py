@@ -202,7 +202,9 @@ def nsa_forward(Q: Tensor, K: Tensor, V: Tensor, cfg, *, gate_logits: Optional[T
         raise NotImplementedError("nsa_forward: pool='learned' is forward-only here (no gradient kernels for the pooling weights)")
     if needs_grad:
         geometry = _geometry(cfg, float(scale), stride_c)
-        ops._check_forward(Q, K, V, gate_logits, False)
+        ops._check_forward(Q, K, V, gate_logits, block_indices, False)
+        if gate_logits is not None and gate_logits.dtype not in (Q.dtype, torch.float32):
+            raise TypeError("nsa_forward: with gradients, gate logits must have Q's dtype or fp32")
         if ops.bwd_engine() != L.ENGINE_GENERIC:
             idx = None if block_indices is None else block_indices.to(torch.int32).contiguous()
             plan = ops.forward_plan(Q.shape, K.shape, Q.dtype, idx_shape=None if idx is None else idx.shape,

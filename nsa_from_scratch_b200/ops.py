@@ -342,8 +342,8 @@ def _plan_forward(key, scales, q_shape, k_shape, dtype, *, causal, cmp_block, cm
     return plan
 
 
-def _check_forward(Q: Tensor, K: Tensor, V: Tensor, gates: Optional[Tensor], token_major: bool) -> None:
-    _need_cuda(Q, K, V)
+def _check_forward(Q: Tensor, K: Tensor, V: Tensor, gates: Optional[Tensor], idx: Optional[Tensor], token_major: bool) -> None:
+    _need_cuda(Q, K, V, gates, idx)
     if V.shape != K.shape:
         raise ValueError(f"K/V shapes {tuple(K.shape)}/{tuple(V.shape)} do not match Q {tuple(Q.shape)}")
     if V.dtype != Q.dtype or K.dtype != Q.dtype:
@@ -359,7 +359,7 @@ def forward(Q: Tensor, K: Tensor, V: Tensor, *, idx: Optional[Tensor] = None, ga
             k_scale: float = 1.0, v_scale: float = 1.0, engine: Optional[int] = None, token_major: bool = False, **geometry) -> Tensor:
     """The whole forward (window means, selection unless `idx` is given, the fused launch) as one library call.
     `geometry`: causal, scale, cmp_block, cmp_stride, bm, bn, window, top_k, force_first, force_local, per_group, gate_act."""
-    _check_forward(Q, K, V, gates, token_major)
+    _check_forward(Q, K, V, gates, idx, token_major)
     Q, K, V = _dense(Q, "Q"), _dense(K, "K"), _dense(V, "V")
     if idx is not None:
         idx = idx.to(torch.int32).contiguous()

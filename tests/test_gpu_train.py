@@ -113,3 +113,21 @@ def test_a_window_beyond_the_sequence(nsa, D):
     assert torch.equal(grads[0][0], grads[1][0])
     for a, b in zip(*(x[1:] for x in grads)):
         assert float((a.float() - b.float()).norm() / a.float().norm()) <= 1e-3
+
+
+def test_refused_gate_logits_and_lists(nsa):
+    """What the kernels cannot read is refused before anything is launched."""
+    Q, K, V, g = make_qkv(29, 1, 2, 1, 128, 128, 64)
+    q, k, v = (t.cuda().requires_grad_(True) for t in (Q, K, V))
+    gates = torch.randn(1, 2, 128, 3, generator=g)
+    idx = torch.zeros(1, 1, 2, 1, dtype=torch.int32)
+    cfg = nsa.NSAConfig(top_k=2, window_size=64)
+    for kw in (dict(gate_logits=gates), dict(gate_logits=gates.bfloat16()), dict(block_indices=idx)):
+        with pytest.raises(RuntimeError, match="CUDA tensors"):
+            nsa.nsa_forward(q, k, v, cfg, **kw)
+        with torch.no_grad(), pytest.raises(RuntimeError, match="CUDA tensors"):
+            nsa.nsa_forward(q, k, v, cfg, **kw)
+    with pytest.raises(TypeError):
+        nsa.nsa_forward(q, k, v, cfg, gate_logits=gates.half().cuda())
+    with pytest.raises(ValueError):
+        nsa.nsa_forward(q, k, v, cfg, gate_logits=gates[:, :, :64].cuda())
