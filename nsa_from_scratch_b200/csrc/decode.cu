@@ -518,6 +518,7 @@ static bool decode_plan(const nsa_decode_args& a, DecodePlan& pl) {
   if (!(a.B > 0 && a.H > 0 && a.Hkv > 0 && a.H % a.Hkv == 0 && a.Tq > 0 && a.Tq <= 64 && a.max_len >= a.Tq && a.top_k > 0 && a.top_k <= DC_MAX_K)) return false;
   if (!(a.cmp_block > 0 && a.cmp_stride > 0 && a.cmp_stride <= a.cmp_block && a.window > 0 && a.scale > 0.f)) return false;
   if (a.nc_alloc < 1 || a.nk_alloc < 1 || a.nk_alloc > DC_MAX_NK) return false;
+  if (a.force_first < 0 || a.force_local < 0) return false;        // the general path refuses them
   DecodeParams& p = pl.p;
   p = {};
   p.G = a.H / a.Hkv;

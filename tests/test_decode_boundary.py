@@ -1,0 +1,21 @@
+"""The decoding step's entry: which calls it takes and which it leaves to the general path, decided from the sizes alone."""
+import ctypes as C
+
+from nsa_from_scratch_b200 import _lib as L
+
+
+def _args(**kw):
+    a = L.DecodeArgs(B=1, H=8, Hkv=2, Tq=1, len=900, D=128, max_len=1024, nc_alloc=63, nk_alloc=16, cmp_block=32, cmp_stride=16, bm=64, bn=64,
+                     top_k=16, window=512, force_first=1, force_local=2, per_group=1, gate_act=L.GATE_SIGMOID, dtype=L.BF16, gate_dtype=0, scale=0.1)
+    for k, v in kw.items():
+        setattr(a, k, v)
+    return a
+
+
+def _ws(**kw):
+    return L.load().nsa_decode_ws_bytes(C.byref(_args(**kw)))
+
+
+def test_negative_forced_counts_are_left_to_the_path_that_refuses_them():
+    assert _ws() > 0
+    assert _ws(force_first=-1) == 0 and _ws(force_local=-1) == 0
