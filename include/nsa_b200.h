@@ -241,7 +241,8 @@ int nsa_backward(const nsa_forward_args* args, const void* dO, const void* branc
  * `len` filled positions; K/V [B,Hkv,max_len,D], pooled Kc/Vc [B,Hkv,nc_alloc,D], block means Kb [B,Hkv,nk_alloc,D].
  * Scores, selection, the three branches and the gated combine: what nsa_forward returns for these queries over the
  * filled prefix.  dyn_len != NULL: the length is read on the device (len is then ignored; the grid is sized for
- * max_len), so that a captured step stays valid as the cache grows.  ws: nsa_decode_ws_bytes(&args) bytes,
+ * max_len, and a larger count is read as max_len), so that a captured step stays valid as the cache grows.  nk_alloc
+ * must cover len (max_len with dyn_len).  ws: nsa_decode_ws_bytes(&args) bytes,
  * 256-byte aligned; 0 means that the shape is not taken (D in {64,128}, 16-bit storage, bm = bn = 64, top_k <= 64,
  * at most 64 query rows per KV head): nsa_select_blocks + nsa_attention_fwd serve those. */
 typedef struct nsa_decode_args {

@@ -269,7 +269,8 @@ __device__ void dc_attend(unsigned char* smem, const DecodeParams& p, const T* K
   }
 }
 
-__device__ __forceinline__ int dc_len(const DecodeParams& p) { return p.dyn_len != nullptr ? *p.dyn_len : p.len; }
+// A count on the device is the caller's to keep: one past the allocation reads as a full cache, never outside of it.
+__device__ __forceinline__ int dc_len(const DecodeParams& p) { return p.dyn_len != nullptr ? min(*p.dyn_len, p.max_len) : p.len; }
 
 // Tasks of phase A: [B*Hkv][n_cmp + n_sld] attention, then [lists][n_score] scoring.
 template <typename T, int D, int MT>
@@ -597,10 +598,16 @@ using namespace nsa;
 
 extern "C" {
 
+// Key blocks of the filled length (of a full cache where the length lives on the device) against the block means' allocation:
+// scores, candidates and means are indexed by key block.
+static bool decode_blocks_fit(const nsa_decode_args& a) { return ((long long)(a.dyn_len ? a.max_len : a.len) + 63) / 64 <= a.nk_alloc; }
+
 int64_t nsa_decode_ws_bytes(const nsa_decode_args* a) {
   NSA_REQUIRE(a, NSA_ERR_ARG, "decode: NULL argument block");
   DecodePlan pl;
-  return decode_plan(*a, pl) ? (int64_t)pl.total : 0;
+  if (!decode_plan(*a, pl)) return 0;
+  NSA_REQUIRE(decode_blocks_fit(*a), NSA_ERR_ARG, "decode: %d block means do not cover the cache", a->nk_alloc);
+  return (int64_t)pl.total;
 }
 
 int nsa_decode(const nsa_decode_args* a, nsa_stream_t stream) {
@@ -610,6 +617,7 @@ int nsa_decode(const nsa_decode_args* a, nsa_stream_t stream) {
               "decode: gate dtype %d", a->gate_dtype);
   DecodePlan pl;
   NSA_REQUIRE(decode_plan(*a, pl), NSA_ERR_UNSUPPORTED, "decode: needs D in {64,128}, 64-token blocks, at most 64 listed blocks and 64 query rows per KV head");
+  NSA_REQUIRE(decode_blocks_fit(*a), NSA_ERR_ARG, "decode: %d block means do not cover the cache", a->nk_alloc);
   NSA_REQUIRE(a->ws_bytes >= (int64_t)pl.total && (reinterpret_cast<uintptr_t>(a->ws) & 255) == 0, NSA_ERR_ARG,
               "decode: needs %lld bytes of workspace (256-byte aligned), %lld given", (long long)pl.total, (long long)a->ws_bytes);
   DecodeParams& p = pl.p;

@@ -101,8 +101,10 @@ def _step(q: Tensor, cache: KVCache, gates: Optional[Tensor], scale: float, dyn_
                      0 if gates is None else L.dtype_code(gates.dtype), scale)
     lib = L.load()
     need = lib.nsa_decode_ws_bytes(C.byref(a))
-    if need <= 0:
+    if need == 0:
         return None
+    if need < 0:
+        L.check(int(need), "nsa_decode")
     out = torch.empty((B, H, Tq, D), device=q.device, dtype=q.dtype)
     ws = torch.empty(need, device=q.device, dtype=torch.uint8)
     a.out, a.ws, a.ws_bytes = out.data_ptr(), ws.data_ptr(), need

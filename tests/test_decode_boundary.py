@@ -19,3 +19,13 @@ def _ws(**kw):
 def test_negative_forced_counts_are_left_to_the_path_that_refuses_them():
     assert _ws() > 0
     assert _ws(force_first=-1) == 0 and _ws(force_local=-1) == 0
+
+
+def test_block_means_that_do_not_cover_the_cache_are_an_error():
+    count = C.c_int32(0)
+    dev = C.addressof(count)                                 # not read: sizes decide
+    assert _ws(nk_alloc=15) > 0 and _ws(nk_alloc=14) == -1   # 900 positions: 15 blocks
+    assert _ws(dyn_len=dev) > 0 and _ws(nk_alloc=15, dyn_len=dev) == -1
+    assert b"do not cover" in L.load().nsa_last_error()
+    a = _args(nk_alloc=14, Q=1, K=1, V=1, Kc=1, Vc=1, Kb=1, out=1, ws=256, ws_bytes=1 << 40)
+    assert L.load().nsa_decode(C.byref(a), None) == -1

@@ -74,3 +74,16 @@ def test_graphed_steps_follow_the_cache(nsa):
         out = dec.step()
         cb.append(Kc[:, :, t:t + 1], Vc[:, :, t:t + 1])
         assert max_abs(out, nsa.nsa_decode(Qc[:, :, t:t + 1], cb, nsplit=1)) <= 1e-2
+
+
+def test_a_device_count_past_the_allocation_reads_as_a_full_cache(nsa):
+    from nsa_from_scratch_b200 import decode
+    B, H, Hkv, D, n = 2, 8, 2, 64, 640
+    Q, K, V, _ = make_qkv(3, B, H, Hkv, 1, n, D)
+    cfg = nsa.NSAConfig(block_size_c=32, stride_c=16, top_k=3, window_size=80, force_first=1, force_local=1, select_per_group=True)
+    cache = nsa.KVCache(B, Hkv, D, n, cfg)
+    cache.append(K.cuda(), V.cuda())
+    want = nsa.nsa_decode(Q.cuda(), cache)
+    for count in (n, n + 1, n + 64, 2**31 - 1):
+        dyn = torch.full((1,), count, dtype=torch.int32, device="cuda")
+        assert max_abs(decode._step(Q.cuda(), cache, None, D ** -0.5, dyn), want) <= 1e-3, count
