@@ -89,13 +89,13 @@ def _step(q: Tensor, cache: KVCache, gates: Optional[Tensor], scale: float, dyn_
         raise ValueError(f"nsa_decode: q {tuple(q.shape)} does not match the cache {tuple(cache.K.shape)}")
     if gates is not None and gates.shape != (B, H, Tq, 3):
         raise ValueError(f"gate_logits shape {tuple(gates.shape)} != {(B, H, Tq, 3)}")
-    ops._need_cuda(q)
+    ops._need_cuda(q, gates)
     q = ops._dense(q, "q")
     gates = None if gates is None else ops._dense(gates, "gates")
     kp, vp, kcp, vcp, kbp = cache._ptrs()
     a = L.DecodeArgs(q.data_ptr(), kp, vp, kcp, vcp, kbp, L.ptr(gates), None, None, L.ptr(dyn_len), 0,
                      B, H, Hkv, Tq, cache.length, D, cache.max_len, cache.Kc.shape[2], cache.Kb.shape[2],
-                     cache.bc, cache.stride, cfg.block_size_m, cache.bn, cfg.top_k, cfg.window_size, _cfg(cfg, "force_first", 0),
+                     cache.bc, cache.stride, int(cfg.block_size_m), cache.bn, cfg.top_k, int(cfg.window_size), _cfg(cfg, "force_first", 0),
                      _cfg(cfg, "force_local", 0), int(bool(_cfg(cfg, "select_per_group", False))),
                      L.GATE_SOFTMAX if cfg.gate_activation == "softmax" else L.GATE_SIGMOID, L.dtype_code(q.dtype),
                      0 if gates is None else L.dtype_code(gates.dtype), scale)

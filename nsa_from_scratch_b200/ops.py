@@ -319,13 +319,14 @@ def _plan_forward(key, scales, q_shape, k_shape, dtype, *, causal, cmp_block, cm
         raise ValueError(f"query heads {H} not a multiple of KV heads {Hkv}")
     a = L.ForwardArgs()
     a.B, a.H, a.Hkv, a.Tq, a.Tk, a.D = B, H, Hkv, Tq, Tk, D
-    a.top_k, a.force_first, a.force_local, a.per_group = int(top_k), int(force_first), int(force_local), int(per_group)
+    a.force_first, a.force_local, a.per_group = int(force_first), int(force_local), int(per_group)
     nq, nk = (Tq + bm - 1) // bm, (Tk + bn - 1) // bn
     if idx_shape is not None:
         if len(idx_shape) != 4 or idx_shape[0] != B or idx_shape[1] not in (H, Hkv) or idx_shape[2] != nq:
             raise ValueError(f"block_indices shape {tuple(idx_shape)} does not match (B={B}, H={H}|{Hkv}, nq={nq}, k)")
         a.has_idx, a.Hi, a.top_k = 1, idx_shape[1], idx_shape[3]
     else:
+        a.top_k = int(top_k)                 # of no account beside given lists, where it may be None
         idx_shape = (B, Hkv if per_group else H, nq, min(int(top_k), nk))
     a.cmp_block, a.cmp_stride, a.bm, a.bn, a.window, a.causal = cmp_block, cmp_stride, bm, bn, window, int(causal)
     a.gate_act, a.q_dtype, a.engine = gate_act, L.dtype_code(dtype), engine

@@ -45,3 +45,22 @@ def test_fp8_forward_with_an_updated_scale_tensor():
     for value in (0.5, 2.0):
         s.fill_(value)
         assert torch.equal(nsa.nsa_forward_fp8(q, k, v, s, s, s, cfg), nsa.nsa_forward_fp8(q, k, v, value, value, value, cfg))
+
+
+def test_given_lists_need_no_top_k():
+    plan = ops.forward_plan(*SHAPES, scale=0.125, q_scale=1.0, k_scale=1.0, v_scale=1.0,
+                            **{**GEOMETRY, "top_k": None, "idx_shape": torch.Size((1, 2, 4, 3))})
+    assert (plan[0].has_idx, plan[0].Hi, plan[0].top_k) == (1, 2, 3)
+
+
+@pytest.mark.gpu
+def test_decoding_takes_a_window_of_another_number_type():
+    import nsa_from_scratch_b200 as nsa
+    g = torch.Generator(device="cuda").manual_seed(6)
+    q, k, v = (torch.randn((1, h, t, 64), generator=g, device="cuda").bfloat16() for h, t in ((4, 1), (2, 300), (2, 300)))
+    outs = []
+    for window in (100, 100.0):
+        cache = nsa.KVCache(1, 2, 64, 320, nsa.NSAConfig(top_k=2, window_size=window))
+        cache.append(k, v)
+        outs.append(nsa.nsa_decode(q, cache))
+    assert torch.equal(*outs)
