@@ -131,7 +131,8 @@ static int n_windows(int T, int block, int stride) {
   return stride == block ? (T + block - 1) / block : (T >= block ? (T - block) / stride + 1 : 0);
 }
 
-// Jobs of one element type and one D; empty ones are dropped.
+// Jobs of one element type and one D; empty ones are dropped.  The kernel counts a job's results in 32 bits: one with 2^31 of
+// them (34 GB) goes in several launches of as many slabs as fit.
 int pool_mean_multi(const PoolJob* jobs, int n_jobs, int D, int dtype, cudaStream_t st) {
   NSA_REQUIRE(D % 8 == 0 && D > 0, NSA_ERR_ARG, "pool: D %d must be a positive multiple of 8", D);
   PoolJobs p;
@@ -144,8 +145,21 @@ int pool_mean_multi(const PoolJob* jobs, int n_jobs, int D, int dtype, cudaStrea
                 n_windows(jb.T, jb.block, jb.stride));
     if (jb.n_out == 0 || jb.slabs == 0) continue;
     NSA_REQUIRE((long long)jb.slabs <= 65535, NSA_ERR_ARG, "pool: B*H %lld too large", (long long)jb.slabs);
-    const long long threads = (long long)jb.slabs * jb.n_out * (D / 8);
-    NSA_REQUIRE(threads < (1LL << 31), NSA_ERR_ARG, "pool: %lld results do not fit a launch", threads);
+    const long long per_slab = (long long)jb.n_out * (D / 8), threads = jb.slabs * per_slab;
+    NSA_REQUIRE(per_slab < (1LL << 31), NSA_ERR_ARG, "pool: %lld results of a head do not fit a launch", per_slab);
+    if (threads >= (1LL << 31)) {
+      const int fit = (int)(((1LL << 31) - 1) / per_slab);
+      const size_t isz = (dtype == NSA_FP8_E4M3 || dtype == NSA_FP8_E5M2) ? 1 : 2;
+      for (int s0 = 0; s0 < jb.slabs; s0 += fit) {
+        PoolJob part = jb;
+        part.x = static_cast<const unsigned char*>(jb.x) + (size_t)s0 * jb.T * D * isz;
+        part.out = static_cast<unsigned char*>(jb.out) + (size_t)s0 * jb.n_out * D * 2;
+        part.slabs = jb.slabs - s0 < fit ? jb.slabs - s0 : fit;
+        const int rc = pool_mean_multi(&part, 1, D, dtype, st);
+        if (rc != NSA_OK) return rc;
+      }
+      continue;
+    }
     p.j[p.n] = jb;
     p.j[p.n].block0 = (unsigned)blocks;
     ++p.n;

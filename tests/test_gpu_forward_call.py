@@ -44,3 +44,20 @@ def test_one_call_equals_the_steps(nsa, H, Hkv, T, Tq, D, group):
                                 gates=gates, gate_act=L.GATE_SIGMOID)
     assert torch.equal(nsa.nsa_forward(Q, K, V, cfg, gate_logits=gates), want)
     assert torch.equal(nsa.nsa_forward(Q, K, V, cfg, gate_logits=gates, block_indices=idx), want)
+
+
+def test_window_means_of_more_results_than_a_launch_counts(nsa):
+    """2^31 results of 8 columns and some more, in pieces of whole heads: every head marked, the ends of each piece compared."""
+    from nsa_from_scratch_b200 import ops
+    T, D, heads = 65536, 128, 2049
+    if torch.cuda.mem_get_info()[0] < 60e9:
+        pytest.skip("needs 52 GB of device memory")
+    x = torch.zeros((1, heads, T, D), dtype=torch.uint8, device="cuda").view(torch.float8_e4m3fn)
+    x.view(torch.uint8)[0, :, 0, 0] = torch.arange(heads, device="cuda").remainder(100).to(torch.uint8)     # finite bit patterns
+    x.view(torch.uint8)[0, :, T - 1, D - 1] = 0x38                                                          # 1.0
+    got = ops.pool_mean(x, 1, 1)
+    assert torch.equal(got[0, :, 0, 0], x[0, :, 0, 0].float().bfloat16())
+    assert bool((got[0, :, T - 1, D - 1] == 1.0).all())
+    assert int((got[0, 2040:] != 0).sum()) == int((x[0, 2040:].view(torch.uint8) != 0).sum())
+    del x, got
+    torch.cuda.empty_cache()
