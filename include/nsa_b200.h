@@ -265,7 +265,7 @@ int nsa_decode(const nsa_decode_args* args, nsa_stream_t stream);
 int nsa_device_status(nsa_stream_t stream);
 
 /* Test hook: writes `value` into the device status word of a kernel family (0 = attention forward,
- * 2 = attention backward) from the host, as a kernel does when one of its bounded waits expires; the
+ * 2 = selected backward, 3 = whole forward's backward) from the host, as a kernel does when one of its bounded waits expires; the
  * next nsa_device_status() must then report NSA_ERR_DEVICE and clear it.  Lets the error path be
  * exercised without making any kernel wait.  No counterpart in the reference. */
 int nsa_debug_set_device_status(int kernel_family, int value);

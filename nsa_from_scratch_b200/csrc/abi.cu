@@ -32,6 +32,7 @@ bool attention_bwd_tc5_supports(const nsa_bwd_args&);
 long long attention_bwd_tc5_scratch_bytes(const nsa_bwd_args&);
 int attention_bwd_tc5(const nsa_bwd_args&, void*, long long, bool, cudaStream_t);
 int bst_take_status(int*);
+int bst_set_status(int);
 int bw5_take_status(int*);
 int tc5_set_status(int);
 int bw5_set_status(int);
@@ -212,8 +213,9 @@ int nsa_device_status(nsa_stream_t stream) {
 }
 
 int nsa_debug_set_device_status(int kernel_family, int value) {
-  NSA_REQUIRE(kernel_family == 0 || kernel_family == 2, NSA_ERR_ARG, "debug status: kernel family %d (0 = forward, 2 = backward)", kernel_family);
-  return kernel_family == 0 ? tc5_set_status(value) : bw5_set_status(value);
+  NSA_REQUIRE(kernel_family == 0 || kernel_family == 2 || kernel_family == 3, NSA_ERR_ARG,
+              "debug status: kernel family %d (0 = forward, 2 = selected backward, 3 = whole forward's backward)", kernel_family);
+  return kernel_family == 0 ? tc5_set_status(value) : (kernel_family == 2 ? bw5_set_status(value) : bst_set_status(value));
 }
 
 int launch_selected_attn_fwd(const void* Q, const void* K, const void* V, const int* Idx, void* Out, float* Lse, int BH,

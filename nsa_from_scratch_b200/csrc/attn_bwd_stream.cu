@@ -884,4 +884,9 @@ int bst_take_status(int* status) {
   return NSA_OK;
 }
 
+int bst_set_status(int v) {
+  NSA_CUDA_OK(cudaMemcpyToSymbol(g_bst_status, &v, sizeof(int)));
+  return NSA_OK;
+}
+
 }  // namespace nsa

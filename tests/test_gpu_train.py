@@ -131,3 +131,13 @@ def test_refused_gate_logits_and_lists(nsa):
         nsa.nsa_forward(q, k, v, cfg, gate_logits=gates.half().cuda())
     with pytest.raises(ValueError):
         nsa.nsa_forward(q, k, v, cfg, gate_logits=gates[:, :, :64].cuda())
+
+
+def test_the_status_word_reaches_the_host(nsa):
+    from nsa_from_scratch_b200 import _lib as L, ops
+    lib = L.load()
+    ops.device_status()
+    assert lib.nsa_debug_set_device_status(3, 5) == 0
+    with pytest.raises(RuntimeError, match="barrier 304"):
+        ops.device_status()
+    ops.device_status()                                    # the report clears it
