@@ -62,11 +62,9 @@ struct Tc5Params {
   int psum;        // one-item kernel, unsplit 16-bit launches: 32 KB of shared memory hold the first 64 columns of the rows' running gated sum
 };
 
-struct Tile {
+struct Tile {     // chunks of a step, and the first key of each
   int nch;
   int j0[2];
-  int jlim[2];
-  int mask[2];   // which of the 4 row groups attend the chunk (selected branch; 0xF otherwise)
 };
 
 // Row maximum (raw scores) of the 32 * NG columns a softmax thread holds: four chains of 3-input max.
@@ -409,10 +407,9 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
     tl.nch = min(2, nchunks[br] - 2 * t);
     for (int c = 0; c < 2; ++c) {
       int ci = min(2 * t + c, nchunks[br] - 1);
-      tl.mask[c] = 0xF;
-      if (br == 0) { tl.j0[c] = ci * 64; tl.jlim[c] = a.Nc; }
-      else if (br == 1) { int blk = sel_list[ci]; tl.j0[c] = blk * 64; tl.jlim[c] = min(blk * 64 + 64, SEL_LIMIT()); tl.mask[c] = sel_mask[ci]; }
-      else { tl.j0[c] = (sld_c0 + ci) * 64; tl.jlim[c] = a.Tk; }
+      if (br == 0) tl.j0[c] = ci * 64;
+      else if (br == 1) tl.j0[c] = sel_list[ci] * 64;
+      else tl.j0[c] = (sld_c0 + ci) * 64;
     }
     return tl;
   };
@@ -456,24 +453,7 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
         const CUtensorMap* mv = br == 0 ? &p.tmVc : &p.tmV;
         const bool raw8 = IN8 && br != 0 && p.kv8;   // pooled K/V of the compressed branch are 16-bit already
         for (int t = tbeg(br); t < tend(br) && ok; ++t, ++it) {
-          const Tile tl = get_tile(br, t);
           const int s = it & 1, ph = (it >> 1) & 1;
-          if (raw8) {
-            // fp8 K/V: TMA fills the staging buffers; the converter warps own the ring slots
-            for (int side = 0; side < 2 && ok; ++side) {
-              ok = __all_sync(0xffffffffu, mbar_wait(bar(B_STGEMPTY + side), (u8 - 1) & 1, &abort_flag));
-              if (!ok) { fail_id = B_STGEMPTY + side + 1; break; }
-              if (leader) {
-                mbar_expect_tx(bar(B_STGFULL + side), (uint32_t)tl.nch * 64 * D);
-                for (int c = 0; c < tl.nch; ++c)
-                  tma_load_3d(smem_u32(stg) + side * STG + c * 64 * D, side == 0 ? mk : mv, bar(B_STGFULL + side), 0, tl.j0[c], kv_slab);
-              }
-            }
-            last_u8 = u8;
-            ++u8;
-            __syncwarp();
-            continue;
-          }
           if constexpr (OWN) {
             if (br == 1) {
               // the next listed block of each row group; a group whose list has ended gets block 0, which no row takes
@@ -499,6 +479,23 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_kernel(const __grid_consta
               __syncwarp();
               continue;
             }
+          }
+          const Tile tl = get_tile(br, t);
+          if (raw8) {
+            // fp8 K/V: TMA fills the staging buffers; the converter warps own the ring slots
+            for (int side = 0; side < 2 && ok; ++side) {
+              ok = __all_sync(0xffffffffu, mbar_wait(bar(B_STGEMPTY + side), (u8 - 1) & 1, &abort_flag));
+              if (!ok) { fail_id = B_STGEMPTY + side + 1; break; }
+              if (leader) {
+                mbar_expect_tx(bar(B_STGFULL + side), (uint32_t)tl.nch * 64 * D);
+                for (int c = 0; c < tl.nch; ++c)
+                  tma_load_3d(smem_u32(stg) + side * STG + c * 64 * D, side == 0 ? mk : mv, bar(B_STGFULL + side), 0, tl.j0[c], kv_slab);
+              }
+            }
+            last_u8 = u8;
+            ++u8;
+            __syncwarp();
+            continue;
           }
           const uint32_t bytes = (uint32_t)tl.nch * 64 * D * 2;
           ok = __all_sync(0xffffffffu, mbar_wait(bar(B_KEMPTY + s), ph ^ 1, &abort_flag));
@@ -1145,10 +1142,9 @@ __global__ void __launch_bounds__(384, 1) nsa_fwd_tc5_persist_kernel(const __gri
     tl.nch = min(2, it.nchunks[br] - 2 * t);
     for (int c = 0; c < 2; ++c) {
       int ci = min(2 * t + c, it.nchunks[br] - 1);
-      tl.mask[c] = 0xF;
-      if (br == 0) { tl.j0[c] = ci * 64; tl.jlim[c] = a.Nc; }
-      else if (br == 1) { int blk = sel_list[lp][ci]; tl.j0[c] = blk * 64; tl.jlim[c] = min(blk * 64 + 64, a.sel_key_limit); tl.mask[c] = sel_mask[lp][ci]; }
-      else { tl.j0[c] = (it.sld_c0 + ci) * 64; tl.jlim[c] = a.Tk; }
+      if (br == 0) tl.j0[c] = ci * 64;
+      else if (br == 1) tl.j0[c] = sel_list[lp][ci] * 64;
+      else tl.j0[c] = (it.sld_c0 + ci) * 64;
     }
     return tl;
   };
