@@ -153,7 +153,7 @@ class _NSAFn(torch.autograd.Function):
     @torch.autograd.function.once_differentiable
     def backward(ctx, grad_out):
         Q, K, V, gates, branch, lse, idx, pooled = ctx.saved_tensors
-        dO = ops._dense(grad_out.to(Q.dtype), "dO")
+        dO = grad_out.to(Q.dtype).contiguous()             # autograd chose its layout (expanded under a sum), not the caller
         dQ, dK, dV, dg = ops.backward(dO, Q, K, V, gates, branch, lse, idx, pooled, ctx.plan)
         return dQ, dK, dV, dg, None, None
 

@@ -141,3 +141,20 @@ def test_the_status_word_reaches_the_host(nsa):
     with pytest.raises(RuntimeError, match="barrier 304"):
         ops.device_status()
     ops.device_status()                                    # the report clears it
+
+
+def test_strict_layout_is_about_the_callers_tensors(nsa):
+    """out.sum() sends back an expanded gradient and a transpose a strided one: no copy that a caller could avoid."""
+    from nsa_from_scratch_b200 import ops
+    Q, K, V, g = make_qkv(37, 1, 2, 1, 128, 128, 64)
+    cfg = nsa.NSAConfig(top_k=2, window_size=64)
+    leaves = [t.cuda().requires_grad_(True) for t in (Q, K, V)]
+    dO = torch.randn(1, 128, 2, 64, generator=g).bfloat16().cuda()
+    ops.set_strict_layout(True)
+    try:
+        one = torch.autograd.grad(nsa.nsa_forward(*leaves, cfg).sum(), leaves)[0]
+        swapped = torch.autograd.grad(nsa.nsa_forward(*leaves, cfg).transpose(1, 2), leaves, dO)[0]
+    finally:
+        ops.set_strict_layout(False)
+    assert torch.equal(one, torch.autograd.grad(nsa.nsa_forward(*leaves, cfg), leaves, torch.ones_like(leaves[0]))[0])
+    assert torch.equal(swapped, torch.autograd.grad(nsa.nsa_forward(*leaves, cfg), leaves, dO.transpose(1, 2).contiguous())[0])
