@@ -61,3 +61,31 @@ def test_window_means_of_more_results_than_a_launch_counts(nsa):
     assert int((got[0, 2040:] != 0).sum()) == int((x[0, 2040:].view(torch.uint8) != 0).sum())
     del x, got
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("H,Hkv,D,group", [(4, 4, 64, False), (4, 1, 128, True), (2, 1, 32, True)])
+@pytest.mark.parametrize("Tk,Tq", [(1, 1), (15, 7), (31, 31)])
+def test_sequences_shorter_than_one_pooling_window(nsa, H, Hkv, D, group, Tk, Tq):
+    """No pooled token: the compressed branch gives nothing, the others their own; against the oracle (2e-2, 16-bit outputs)."""
+    from helpers import make_qkv, max_abs
+    from oracle import nsa_oracle as O
+    Q, K, V, g = make_qkv(5, 2, H, Hkv, Tq, Tk, D)
+    gates = torch.randn(2, H, Tq, 3, generator=g)
+    cfg = nsa.NSAConfig(block_size_c=32, stride_c=16, top_k=2, window_size=8, select_per_group=group)
+    idx = O.select_blocks(Q, K, top_k=2, group_shared=group)
+    gv = torch.sigmoid(gates)
+    ref = gv[..., 1:2] * O.selected_attention(Q, K, V, block_indices=idx)[0] + gv[..., 2:3] * O.sliding_attention(Q, K, V, window_size=8)[0]
+    out = nsa.nsa_forward(Q.cuda(), K.cuda(), V.cuda(), cfg, gate_logits=gates.cuda())
+    assert max_abs(out, ref) <= 2e-2
+
+
+@pytest.mark.parametrize("bm,bn,k", [(64, 32, 3), (128, 128, 2), (64, 64, 70)])
+def test_fp8_beyond_the_tcgen05_kernels_shapes(nsa, bm, bn, k):
+    """The generic kernel converts as it loads: bit-equal to the same call on the dequantised tensors."""
+    g = torch.Generator().manual_seed(7)
+    T = 70 * 64 + 5 if k == 70 else 300
+    q8, k8, v8 = (torch.randn(1, h, T, 64, generator=g).to(torch.float8_e4m3fn).cuda() for h in (2, 1, 1))
+    cfg = nsa.NSAConfig(block_size_c=32, stride_c=16, block_size_m=bm, block_size_n=bn, top_k=k, window_size=65, select_per_group=True)
+    s = 0.37
+    want = nsa.nsa_forward(*((x.float() * s).bfloat16() for x in (q8, k8, v8)), cfg)
+    assert torch.equal(nsa.nsa_forward_fp8(q8, k8, v8, s, s, s, cfg), want)
