@@ -1863,6 +1863,7 @@ bool attention_fwd_tc5_supports(const nsa_fwd_args& a) {
 // 2.72, sliding 1.93 against 2.02); launches of several branches are 1-4 % slower on it than on the one-item kernel
 // (all three: 8.91-9.25 against 8.54-8.89 ms on the same box) and stay there, as do the split and fp8 launches.
 // NSA_TC5_PERSIST=0 / =1 in the environment forces the one-item / the persistent kernel for every unsplit 16-bit launch.
+// The launch whose log-sum-exp the block scores are formed with is on the persistent kernel in any case.
 static int tc5_persistent_mode() {
   static const int mode = [] { const char* e = getenv("NSA_TC5_PERSIST"); return !e ? -1 : (e[0] == '0' ? 0 : 1); }();
   return mode;
